@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 
+#include "gemm_rns.cuh"
 #include "gemm_tc.cuh"
 #include "op_internal.h"
 
@@ -36,6 +37,12 @@ int fail(bg_ctx* ctx, int code, const std::string& msg) {
 
 int cuda_fail(bg_ctx* ctx, cudaError_t e, const char* what) {
   return fail(ctx, BG_EDEVICE, std::string(what) + ": " + cudaGetErrorString(e));
+}
+
+int report_error_bits(bg_ctx* ctx, int bits) {
+  if (bits & rns::kErrBit) return fail(ctx, BG_ETIMEOUT, "tensor-core product: a pipeline wait gave up");
+  if (bits) return fail(ctx, BG_ENONFINITE, (bits & 2) ? "non-finite potential value" : "non-finite input coefficient");
+  return BG_OK;
 }
 }  // namespace bg
 
@@ -159,6 +166,38 @@ int ksplit_tiles(int64_t rows, int64_t tiles, int* kchunk, int64_t ks_cap = 1 <<
 
 int ksplit_for(int64_t rows, int nproj, int64_t cols, int* kchunk) {
   return ksplit_tiles(rows, (int64_t)((nproj + 47) / 48) * ((cols + 47) / 48), kchunk);
+}
+
+// The projector table as residue panels of the FP64 products (gemm_rns.cuh), constant for
+// the operator's lifetime.  Without memory for them the operator keeps the FP64 tiles.
+int residue_panels(bg_op* op, const double2* p, int nproj) {
+  NlDev& N = op->nl;
+  const int rows = (int)op->rows;
+  const size_t bytes[4] = {rns::a_panel_bytes(nproj, rows), rns::a_panel_bytes(rows, nproj),
+                           2 * sizeof(double) * (size_t)nproj, 2 * sizeof(double) * (size_t)rows};
+  std::unique_ptr<DevBuf> b[4];
+  for (int i = 0; i < 4; ++i) {
+    b[i] = std::make_unique<DevBuf>();
+    b[i]->bytes = bytes[i];
+    if (cudaMalloc(&b[i]->p, bytes[i]) != cudaSuccess) {
+      b[i]->p = nullptr;
+      cudaGetLastError();
+      return BG_OK;
+    }
+  }
+  auto* tn = static_cast<unsigned char*>(b[0]->p);
+  auto* nn = static_cast<unsigned char*>(b[1]->p);
+  auto* tn_scale = static_cast<double*>(b[2]->p);
+  auto* nn_scale = static_cast<double*>(b[3]->p);
+  cudaError_t e = rns::split_a(rns::kTN, p, rows, nproj, rows, tn, tn_scale, tn_scale + nproj, nullptr);
+  if (e == cudaSuccess) e = rns::split_a(rns::kNN, p, rows, rows, nproj, nn, nn_scale, nn_scale + rows, nullptr);
+  if (e != cudaSuccess) return cuda_fail(op->ctx, e, "projector residues");
+  N.r_tn = tn;
+  N.r_nn = nn;
+  N.r_tn_inv = tn_scale + nproj;
+  N.r_nn_inv = nn_scale + rows;
+  for (auto& x : b) op->bufs.push_back(std::move(x));
+  return BG_OK;
 }
 
 // Build the stick plan, the tables and the nonlocal operands of one operator.
@@ -465,6 +504,7 @@ int build_op(bg_ctx* ctx, const bg_basis_desc* b, const bg_projectors* pr, int64
       if (ce == cudaSuccess)
         ce = tc::split_a(tc::kNN, pd, npw, (int)npw, nproj, const_cast<unsigned char*>(N.p_nn), nullptr);
       if (ce != cudaSuccess) return cuda_fail(ctx, ce, "projector panels");
+      if (rns::pays(nproj, capacity, npw, true) && (rc = residue_panels(op.get(), pd, nproj))) return rc;
     }
     N.p = d_dbl;
     op->shape.natoms = natoms;
@@ -515,7 +555,8 @@ int build_op(bg_ctx* ctx, const bg_basis_desc* b, const bg_projectors* pr, int64
 }
 
 // Wait for the operator stream and report (then clear) the device error word:
-// bit 0 a non-finite coefficient read by a kernel, bit 1 a non-finite potential value.
+// bit 0 a non-finite coefficient read by a kernel, bit 1 a non-finite potential value,
+// bit 2 (rns::kErrBit) a bounded device wait that gave up.
 int check_err(bg_op* op) {
   cudaError_t e = cudaMemcpyAsync(op->err_host, op->t.err, sizeof(int), cudaMemcpyDeviceToHost, op->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(op->stream);
@@ -524,7 +565,7 @@ int check_err(bg_op* op) {
   if (bits) {
     cudaMemsetAsync(op->t.err, 0, sizeof(int), op->stream);
     cudaStreamSynchronize(op->stream);
-    return fail(op->ctx, BG_ENONFINITE, (bits & 2) ? "non-finite potential value" : "non-finite input coefficient");
+    return report_error_bits(op->ctx, bits);
   }
   return BG_OK;
 }
@@ -614,6 +655,7 @@ int bg_op_destroy(bg_op* op) {
   if (op->own_stream && op->stream) cudaStreamDestroy(op->stream);
   if (op->err_host) cudaFreeHost(op->err_host);
   op->tc.release();
+  op->rns.release();
   delete op;
   return BG_OK;
 }
@@ -691,6 +733,10 @@ int bg_op_apply_block(bg_op* op, const double* x, double* y, int64_t rows, int64
                                precision != BG_PREC_FP64 ? 1 : 0);
   if (tensor_nl) {
     op->launches += launch_nonlocal_tc(op->d_nl, op->shape, (int)op->rows, (int)cols, bt, &op->tc, op->stream, &op->ev);
+  } else if (op->shape.nproj > 0 && op->nl.r_tn && rns::pays(op->shape.nproj, cols, op->rows, true) &&
+             ensure_nonlocal_rns(&op->rns, 1, op->shape.nproj, op->cap, (int)op->rows, op->stream)) {
+    op->launches += launch_nonlocal_rns(op->d_nl, op->shape, (int)op->rows, (int)cols, bt, &op->rns, op->t.err,
+                                        op->stream, &op->ev);
   } else if (op->shape.nproj > 0) {
     NlShape sh = op->shape;
     sh.ksplit = ksplit_for(op->rows, sh.nproj, cols, &sh.kchunk);
@@ -938,8 +984,20 @@ int ensure_potential_float(bg_op* op, cudaStream_t s) {
   return BG_OK;
 }
 
+// Whether the nonlocal products of operators [k0, k1) run as residue products: every
+// operator has its panels, the widest block pays, and the buffers (sized for the whole
+// set's capacities) are there.
+static bool residue_products(bg_kset* ks, int k0, int k1, int64_t max_cols, int max_rows, RnsNl* r, cudaStream_t s) {
+  if (ks->gamma || ks->shape.nproj == 0 || !rns::pays(ks->shape.nproj, max_cols, max_rows, true)) return false;
+  for (int k = k0; k < k1; ++k)
+    if (!ks->ops[k]->nl.r_tn) return false;
+  int64_t cap = 0;
+  for (const bg_op* o : ks->ops) cap = std::max(cap, o->cap);
+  return ensure_nonlocal_rns(r, (int)ks->ops.size(), ks->shape.nproj, cap, ks->max_rows, s);
+}
+
 int enqueue_range(bg_kset* ks, int k0, int k1, const CallArgs* args, const int64_t* cols, cudaStream_t s,
-                  StageEvents* ev, int prec, TcNl* tc) {
+                  StageEvents* ev, int prec, TcNl* tc, RnsNl* rns) {
   Batch bt;
   bt.nk = k1 - k0;
   int max_groups = 0, max_rows = 0;
@@ -954,6 +1012,9 @@ int enqueue_range(bg_kset* ks, int k0, int k1, const CallArgs* args, const int64
   int launches = launch_local(ks->d_tabs + k0, ks->gamma, max_groups, ks->g, bt, s, ev, prec != BG_PREC_FP64 ? 1 : 0);
   if (prec == BG_PREC_TENSOR && !ks->gamma && ks->shape.nproj > 0) {
     launches += launch_nonlocal_tc(ks->d_nl + k0, ks->shape, max_rows, (int)max_cols, bt, tc ? tc : &ks->tc, s, ev);
+  } else if (residue_products(ks, k0, k1, max_cols, max_rows, rns ? rns : &ks->rns, s)) {
+    launches += launch_nonlocal_rns(ks->d_nl + k0, ks->shape, max_rows, (int)max_cols, bt, rns ? rns : &ks->rns,
+                                    ks->ops[k0]->t.err, s, ev);
   } else if (ks->shape.nproj > 0) {
     NlShape sh = ks->shape;
     int64_t tiles = 0, cap = 1 << 30;
@@ -1052,6 +1113,7 @@ int bg_kset_destroy(bg_kset* ks) {
   cudaFree(ks->d_tabs);
   cudaFree(ks->d_nl);
   ks->tc.release();
+  ks->rns.release();
   delete ks;
   return BG_OK;
 }
@@ -1428,7 +1490,7 @@ int bg_kset_sync(bg_kset* ks) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(ks->stream);
   if (e != cudaSuccess) return cuda_fail(ks->ctx, e, "k-point set");
   for (int k = 0; k < n; ++k)
-    if (ks->h_errv[k]) return fail(ks->ctx, BG_ENONFINITE, "non-finite input coefficient");
+    if (ks->h_errv[k]) return report_error_bits(ks->ctx, ks->h_errv[k]);
   return BG_OK;
 }
 

@@ -111,6 +111,12 @@ struct NlDev {
   const unsigned char* p_tn;
   const unsigned char* p_nn;
   int kt_tn, kt_nn;
+  // and, where the operator's products are large enough, as int8 residue panels of the FP64
+  // products (gemm_rns.cuh) with the inverse scales of their rows; null otherwise
+  const unsigned char* r_tn;
+  const unsigned char* r_nn;
+  const double* r_tn_inv;
+  const double* r_nn_inv;
 };
 
 struct NlShape {
@@ -156,6 +162,25 @@ int ensure_nonlocal_tc(TcNl* tc, int nk, int nproj, int max_cols, int max_rows);
 // coupling D in FP64); complex operators only.
 int launch_nonlocal_tc(const NlDev* nl, const NlShape& sh, int max_rows, int max_cols, const Batch& b, TcNl* tc,
                        cudaStream_t s, StageEvents* ev);
+
+// Buffers of the FP64 nonlocal products on the int8 tensor cores (gemm_rns.cuh): the
+// descriptors of a batch (2 kMaxBatch) and one workspace, allocated once at the size of the
+// batch's largest blocks and never moved (captured graphs may hold their addresses).
+struct RnsNl {
+  void* desc = nullptr;
+  void* work = nullptr;
+  size_t bytes = 0;
+  bool tried = false;
+  void release();
+};
+// True when the buffers are ready for blocks of up to max_cols columns (the same bound on
+// every call).  Allocates on the first call outside a stream capture; a failed allocation
+// leaves the FP64 tiles in use.
+bool ensure_nonlocal_rns(RnsNl* r, int nk, int nproj, int64_t max_cols, int max_rows, cudaStream_t s);
+// Enqueue y += P (D (P^H x)) with both products as residue products (complex operators
+// with panels); err: the device error word of a wait that gave up.
+int launch_nonlocal_rns(const NlDev* nl, const NlShape& sh, int max_rows, int max_cols, const Batch& b, RnsNl* r,
+                        int* err, cudaStream_t s, StageEvents* ev);
 
 // Band densities of the blocks of a batch (k = 0 .. b.nk - 1, operator tables tabs[k]
 // and their stick buffers): part[k][c][z][y n0 + x] = sum over the units of chunk c of

@@ -20,6 +20,7 @@
 // crates/dft-physics/src/distributed_real_gamma.rs:654-689 (pair pack), :1307-1347
 // (unpack + kinetic), :957-1017, 1184-1248 (nonlocal).
 #include "hpsi.h"
+#include "gemm_rns.cuh"
 #include "gemm_tc.cuh"
 #include "fft_fast.cuh"
 #include "gemm_tiles.cuh"
@@ -1060,6 +1061,74 @@ int ensure_nonlocal_tc(TcNl* t, int nk, int nproj, int max_cols, int max_rows) {
     t->work_bytes = need;
   }
   return 0;
+}
+
+// Descriptors of the FP64 residue products of every operator of a batch: [k] P^H x into the
+// projection buffer, [nk + k] y += P wd.  One thread per operator.
+__global__ void k_nl_rns_descs(const NlDev* __restrict__ nls, int nproj, Batch b, rns::Desc* __restrict__ out) {
+  const int k = threadIdx.x;
+  if (k >= b.nk) return;
+  const NlDev& nl = nls[k];
+  const CallArgs ca = resolve(b.a[k]);
+  const int cols = ca.cols;
+  const double2* p = reinterpret_cast<const double2*>(nl.p);
+  out[k] = rns::Desc{p,     reinterpret_cast<const double2*>(ca.x), reinterpret_cast<double2*>(nl.part), nl.rows,
+                     ca.ldx / 2, nproj, cols > 0 ? nproj : 0, cols, nl.rows, rns::kStore, nl.r_tn, nl.r_tn_inv,
+                     (nl.rows + rns::kTileK - 1) / rns::kTileK};
+  out[b.nk + k] = rns::Desc{p, reinterpret_cast<const double2*>(nl.wd), reinterpret_cast<double2*>(ca.y), nl.rows,
+                            nproj, ca.ldy / 2, cols > 0 ? nl.rows : 0, cols, nproj, rns::kAdd, nl.r_nn, nl.r_nn_inv,
+                            (nproj + rns::kTileK - 1) / rns::kTileK};
+}
+
+void RnsNl::release() {
+  cudaFree(desc);
+  cudaFree(work);
+  desc = work = nullptr;
+}
+
+bool ensure_nonlocal_rns(RnsNl* r, int nk, int nproj, int64_t max_cols, int max_rows, cudaStream_t s) {
+  if (r->work) return true;
+  if (r->tried) return false;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  r->tried = true;
+  // the projection and the back-projection run one after the other on one stream and share
+  // the workspace
+  const size_t need = std::max(rns::workspace_bytes(rns::kTN, nk, nproj, (int)max_cols, max_rows, true),
+                               rns::workspace_bytes(rns::kNN, nk, max_rows, (int)max_cols, nproj, true));
+  if (rns::prepare() != cudaSuccess || cudaMalloc(&r->desc, sizeof(rns::Desc) * 2 * kMaxBatch) != cudaSuccess ||
+      cudaMalloc(&r->work, need) != cudaSuccess) {
+    cudaGetLastError();
+    r->release();
+    return false;
+  }
+  r->bytes = need;
+  return true;
+}
+
+int launch_nonlocal_rns(const NlDev* nl, const NlShape& sh, int max_rows, int max_cols, const Batch& b, RnsNl* r,
+                        int* err, cudaStream_t s, StageEvents* ev) {
+  if (sh.nproj == 0 || max_cols == 0 || b.nk == 0) return 0;
+  rns::Desc* d = static_cast<rns::Desc*>(r->desc);
+  int launches = 2;
+  k_nl_rns_descs<<<1, kMaxBatch, 0, s>>>(nl, sh.nproj, b, d);
+  {
+    StageScope sc(ev, 3, s);
+    launches += rns::launch_product(rns::kTN, d, b.nk, sh.nproj, max_cols, max_rows, true, r->work, r->bytes, err, s);
+  }
+  {
+    StageScope sc(ev, 4, s);
+    const dim3 cg(sh.natoms, max_cols, b.nk);
+    k_couple<double2><<<cg, ((sh.maxch + 31) / 32) * 32, 0, s>>>(nl, sh.nproj, 1, b);
+  }
+  {
+    StageScope sc(ev, 5, s);
+    launches += rns::launch_product(rns::kNN, d + b.nk, b.nk, max_rows, max_cols, sh.nproj, true, r->work, r->bytes, err, s);
+  }
+  return launches;
 }
 
 int launch_nonlocal_tc(const NlDev* nl, const NlShape& sh, int max_rows, int max_cols, const Batch& b, TcNl* t,

@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "blas_dev.cuh"
+#include "gemm_rns.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_tiles.cuh"
 #include "tridiag_dev.cuh"
@@ -572,18 +573,21 @@ __device__ bool eigen(const Bufs<D>& b, int cap, int m, double* red, int* sh) {
 // ------------------------------------------------------------------ batched large products
 // Descriptor arrays are laid out [slot][k]; blockIdx.z enumerates (slot, k).
 
-// C (+)= A B for every (slot, k) with a non-empty descriptor; 64 x 64 tiles.  blockIdx.x
+// C (+)= A B for every (slot, k) with a non-empty descriptor; 64 x 64 tiles.  residues: the
+// launch is paired with one of the residue products (gemm_rns.cuh), which take the products
+// that pay there.  blockIdx.x
 // runs over the column tiles, so the blocks that read one 64-row slice of the tall A
 // launch together and share it in L2.
 template <class D>
 __global__ void __launch_bounds__(256, 2) k_dv_nn(const Bufs<D>* __restrict__ bufs, const NN<D>* __restrict__ desc,
-                                                  int nk) {
+                                                  int nk, int residues) {
   const int z = blockIdx.z, k = z % nk;
   const NN<D> d = desc[z];
   const int rows = bufs[k].rows;
   const int64_t r0 = (int64_t)blockIdx.y * 64;
   const int j0 = blockIdx.x * 64;
   if (d.n <= 0 || d.prec || j0 >= d.n || r0 >= rows) return;
+  if (residues && rns::pays(rows, d.n, d.k, false)) return;  // formed by the residue products
   tiles::nn_tile64_mma<D, true>(d.A, rows, d.B, d.ldb, d.C, rows, rows, d.n, d.k, r0, j0, d.accumulate != 0);
 }
 
@@ -591,12 +595,13 @@ __global__ void __launch_bounds__(256, 2) k_dv_nn(const Bufs<D>* __restrict__ bu
 // conj(A[r][i]) B[r][j]; blockIdx.z = (slot * nk + k) * ks + s.
 template <class D>
 __global__ void __launch_bounds__(256, 2) k_dv_tn(const Bufs<D>* __restrict__ bufs, const TN<D>* __restrict__ desc, int nk,
-                                              int ks, int64_t slot_elems) {
+                                              int ks, int64_t slot_elems, int residues) {
   const int zz = blockIdx.z / ks, sidx = blockIdx.z % ks;
   const int slot = zz / nk, k = zz % nk;
   const TN<D> d = desc[zz];
   if (d.m <= 0 || d.n <= 0 || d.prec || (int)blockIdx.x * 48 >= d.m || (int)blockIdx.y * 48 >= d.n) return;
   const int64_t rows = bufs[k].rows;
+  if (residues && rns::pays(d.m, d.n, rows, false)) return;
   int64_t chunk = (rows + ks - 1) / ks;
   chunk = ((chunk + 31) / 32) * 32;
   const int64_t r0 = min(rows, (int64_t)sidx * chunk), r1 = min(rows, r0 + chunk);
@@ -607,10 +612,10 @@ __global__ void __launch_bounds__(256, 2) k_dv_tn(const Bufs<D>* __restrict__ bu
 // G[i + j ldg] = sum_s part[slot][s][j][i] in slice order.
 template <class D>
 __global__ void k_dv_tn_sum(const Bufs<D>* __restrict__ bufs, const TN<D>* __restrict__ desc, int nk, int ks,
-                            int64_t slot_elems) {
+                            int64_t slot_elems, int residues) {
   const int zz = blockIdx.z, slot = zz / nk, k = zz % nk;
   const TN<D> d = desc[zz];
-  if (d.m <= 0 || d.n <= 0 || d.prec) return;
+  if (d.m <= 0 || d.n <= 0 || d.prec || (residues && rns::pays(d.m, d.n, bufs[k].rows, false))) return;
   const D* part = bufs[k].part + slot * slot_elems;
   const int64_t total = (int64_t)d.m * d.n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
@@ -719,6 +724,32 @@ __global__ void k_dv_tc_descs(const Bufs<D>* __restrict__ bufs, const NN<D>* __r
                     ? tc::ZDesc{reinterpret_cast<const double2*>(d.A), reinterpret_cast<const double2*>(d.B),
                                 reinterpret_cast<double2*>(d.G), rows, rows, d.ldg, d.m, d.n, (int)rows, tc::kStore}
                     : empty;
+  }
+}
+
+// Residue-product descriptors of the FP64 products that pay there (complex blocks): one
+// thread per (slot, k point); the others get empty descriptors.
+template <class D>
+__global__ void k_dv_rns_descs(const Bufs<D>* __restrict__ bufs, const NN<D>* __restrict__ nn, int n_nn,
+                               const TN<D>* __restrict__ tn, int n_tn, int nk, rns::Desc* out) {
+  const int z = blockIdx.x * blockDim.x + threadIdx.x;
+  rns::Desc o{nullptr, nullptr, nullptr, 1, 1, 1, 0, 0, 0, rns::kStore};
+  if (z < n_nn * nk) {
+    const NN<D> d = nn[z];
+    const int64_t rows = bufs[z % nk].rows;
+    if (!d.prec && d.n > 0 && d.k > 0 && rns::pays(rows, d.n, d.k, false))
+      o = rns::Desc{reinterpret_cast<const double2*>(d.A), reinterpret_cast<const double2*>(d.B),
+                    reinterpret_cast<double2*>(d.C), rows, d.ldb, rows, (int)rows, d.n, d.k,
+                    d.accumulate ? rns::kAdd : rns::kStore};
+    out[z] = o;
+  }
+  if (z < n_tn * nk) {
+    const TN<D> d = tn[z];
+    const int64_t rows = bufs[z % nk].rows;
+    if (!d.prec && d.m > 0 && d.n > 0 && rns::pays(d.m, d.n, rows, false))
+      o = rns::Desc{reinterpret_cast<const double2*>(d.A), reinterpret_cast<const double2*>(d.B),
+                    reinterpret_cast<double2*>(d.G), rows, rows, d.ldg, d.m, d.n, (int)rows, rns::kStore};
+    out[z] = o;
   }
 }
 
@@ -1397,6 +1428,7 @@ class KsetSolver {
   }
   ~KsetSolver() {
     tcnl_.release();
+    rnsnl_.release();
     for (int p = 0; p < 3; ++p) {
       if (exec_[p]) cudaGraphExecDestroy(exec_[p]);
       if (graph_[p]) cudaGraphDestroy(graph_[p]);
@@ -1425,6 +1457,12 @@ class KsetSolver {
   int* tc_err_ = nullptr;
   int tc_ks_ = 1;
   bool tc_ready_ = false;
+  // FP64 products on the int8 tensor cores: the solver's own buffers of the applies'
+  // nonlocal products and of its Grams and rotations (null where no product pays)
+  RnsNl rnsnl_;
+  rns::Desc* d_rns_ = nullptr;
+  unsigned char* rns_work_ = nullptr;
+  size_t rns_bytes_ = 0;
   unsigned* d_bar_ = nullptr;   // grid barrier of the cooperative launches
   double* d_wpart_ = nullptr;   // their per-block partial sums
   int coop_blocks_ = 0;
@@ -1487,26 +1525,72 @@ class KsetSolver {
                                                      nk_, ks_->gamma);
     return 1;
   }
-  int64_t nn(int nslots) {
+  // residues: large products go through the residue products (not in the repair, whose
+  // launches are nearly always empty)
+  int64_t nn(int nslots, bool residues = true) {
     const dim3 grid((unsigned)((o_.cap + 63) / 64), (unsigned)((max_rows_ + 63) / 64), (unsigned)(nslots * nk_));
-    k_dv_nn<D><<<grid, 256, tiles::nn64m_smem_bytes<D>(), s_>>>(d_bufs_, d_nn_, nk_);
-    if (!tensor_products()) return 1;
+    residues = residues && rns_work_;
+    k_dv_nn<D><<<grid, 256, tiles::nn64m_smem_bytes<D>(), s_>>>(d_bufs_, d_nn_, nk_, residues ? 1 : 0);
+    int64_t l = 1;
+    if (residues) {
+      k_dv_rns_descs<D><<<1, 128, 0, s_>>>(d_bufs_, d_nn_, nslots, d_tn_, 0, nk_, d_rns_);
+      l += 1 + rns::launch_product(rns::kNN, d_rns_, nslots * nk_, max_rows_, o_.n, o_.cap, false, rns_work_, rns_bytes_,
+                                   ks_->ops[0]->t.err, s_);
+    }
+    if (!tensor_products()) return l;
     k_dv_tc_descs<D><<<1, 128, 0, s_>>>(d_bufs_, d_nn_, nslots, d_tn_, 0, nk_, d_tcnn_, d_tctn_);
-    return 2 + tc::launch_zgemm(tc::kNN, d_tcnn_, nslots * nk_, max_rows_, o_.cap, o_.cap, 1, false, tc_work_,
+    return l + 1 + tc::launch_zgemm(tc::kNN, d_tcnn_, nslots * nk_, max_rows_, o_.cap, o_.cap, 1, false, tc_work_,
                                 tc_err_, s_);
   }
   bool tensor_products() const { return o_.tensor && sizeof(D) == sizeof(double2) && tc_ready_; }
-  int64_t tn(int nslots) {
+  int64_t tn(int nslots, bool residues = true) {
     const unsigned t = (unsigned)((o_.cap + 47) / 48);
+    residues = residues && rns_work_;
     k_dv_tn<D><<<dim3(t, t, (unsigned)(nslots * nk_ * ksplit_)), 256, tiles::tn48m_smem_bytes<D>(), s_>>>(
-        d_bufs_, d_tn_, nk_, ksplit_, slot_elems_);
+        d_bufs_, d_tn_, nk_, ksplit_, slot_elems_, residues ? 1 : 0);
     const unsigned blocks = (unsigned)std::min<int64_t>(((int64_t)o_.cap * o_.cap + 255) / 256, 64);
     k_dv_tn_sum<D><<<dim3(blocks, 1, (unsigned)(nslots * nk_)), 256, 0, s_>>>(d_bufs_, d_tn_, nk_, ksplit_,
-                                                                              slot_elems_);
-    if (!tensor_products()) return 2;
+                                                                              slot_elems_, residues ? 1 : 0);
+    int64_t l = 2;
+    if (residues) {
+      k_dv_rns_descs<D><<<1, 128, 0, s_>>>(d_bufs_, d_nn_, 0, d_tn_, nslots, nk_, d_rns_);
+      l += 1 + rns::launch_product(rns::kTN, d_rns_, nslots * nk_, o_.cap, o_.n, max_rows_, false, rns_work_, rns_bytes_,
+                                   ks_->ops[0]->t.err, s_);
+    }
+    if (!tensor_products()) return l;
     k_dv_tc_descs<D><<<1, 128, 0, s_>>>(d_bufs_, d_nn_, 0, d_tn_, nslots, nk_, d_tcnn_, d_tctn_);
-    return 3 + tc::launch_zgemm(tc::kTN, d_tctn_, nslots * nk_, o_.cap, o_.cap, max_rows_, tc_ks_, false, tc_work_,
+    return l + 1 + tc::launch_zgemm(tc::kTN, d_tctn_, nslots * nk_, o_.cap, o_.cap, max_rows_, tc_ks_, false, tc_work_,
                                 tc_err_, s_);
+  }
+  // Buffers of the residue products (once, before any capture), where the largest Gram or
+  // rotation pays; without memory for them every product stays on the FP64 tiles.
+  void prepare_residues() {
+    if (sizeof(D) != sizeof(double2)) return;
+    if (!ks_->dense && ks_->shape.nproj > 0 && rns::pays(ks_->shape.nproj, o_.n, max_rows_, true)) {
+      bool panels = true;
+      int64_t cap = 0;
+      for (const bg_op* op : ks_->ops) {
+        panels = panels && op->nl.r_tn;
+        cap = std::max(cap, op->cap);
+      }
+      if (panels) ensure_nonlocal_rns(&rnsnl_, nk_, ks_->shape.nproj, o_.n, max_rows_, s_);
+    }
+    if (2 * nk_ > 128 || !rns::pays(o_.cap, o_.n, max_rows_, false)) return;
+    static_assert(kNnSlots == 2 && kTnSlots == 2, "descriptor slots");
+    const size_t need = std::max(rns::workspace_bytes(rns::kTN, 2 * nk_, o_.cap, o_.n, max_rows_, false),
+                                 rns::workspace_bytes(rns::kNN, 2 * nk_, max_rows_, o_.n, o_.cap, false));
+    void *d = nullptr, *w = nullptr;
+    if (rns::prepare() != cudaSuccess || cudaMalloc(&d, sizeof(rns::Desc) * 2 * nk_) != cudaSuccess ||
+        cudaMalloc(&w, need) != cudaSuccess) {
+      cudaGetLastError();
+      cudaFree(d);
+      return;
+    }
+    dev_.push_back(d);
+    dev_.push_back(w);
+    d_rns_ = static_cast<rns::Desc*>(d);
+    rns_work_ = static_cast<unsigned char*>(w);
+    rns_bytes_ = need;
   }
   // Buffers of the precision form (once, before any capture).
   int prepare_tensor() {
@@ -1557,7 +1641,7 @@ class KsetSolver {
       return 1;
     }
     return enqueue_range(ks_, 0, nk_, args_.data(), cols_.data(), s_, nullptr,
-                         o_.tensor ? BG_PREC_TENSOR : (o_.fp32 ? BG_PREC_FP32 : BG_PREC_FP64), &tcnl_);
+                         o_.tensor ? BG_PREC_TENSOR : (o_.fp32 ? BG_PREC_FP32 : BG_PREC_FP64), &tcnl_, &rnsnl_);
   }
   int64_t iteration() {
     int64_t l = 0;
@@ -1568,11 +1652,11 @@ class KsetSolver {
     l += ctl(kSelect) + cp(0, 1) + tn(1);
     l += ctl(kExtend);
     if (wide_) l += wchol() + ctl(kExtendPost);
-    l += cp(0, 1) + nn(2) + cp(1, 2);
-    l += ctl(kRepair1) + tn(1);
-    l += ctl(kRepair2) + nn(1) + tn(1);
-    l += ctl(kRepair3) + nn(1) + tn(1);
-    l += ctl(kRepair4) + nn(1) + cp(0, 1) + tn(1);
+    l += cp(0, 1) + nn(2, false) + cp(1, 2);
+    l += ctl(kRepair1) + tn(1, false);
+    l += ctl(kRepair2) + nn(1, false) + tn(1, false);
+    l += ctl(kRepair3) + nn(1, false) + tn(1, false);
+    l += ctl(kRepair4) + nn(1, false) + cp(0, 1) + tn(1, false);
     l += ctl(kApply);
     if (wide_) l += wchol() + ctl(kApplyPost);
     l += apply() + tn(1);
@@ -1668,6 +1752,7 @@ int KsetSolver<T>::prepare() {
   }
   if ((rc = cuda(cudaMemcpy(d_bufs_, hb_.data(), sizeof(Bufs<D>) * nk_, cudaMemcpyHostToDevice), "upload")))
     return rc;
+  prepare_residues();
   args_.assign(nk_, CallArgs{});
   cols_.assign(nk_, n);
   for (int k = 0; k < nk_; ++k) {
@@ -1823,8 +1908,14 @@ int KsetSolver<T>::run(const double* const* start, const double* const* diagonal
       return BG_ETIMEOUT;
     }
   }
-  // a non-finite block met by the applies
+  // a residue product's pipeline wait gave up, or a non-finite block met by the applies
   for (int k = 0; k < nk_; ++k) {
+    if ((int)h_out_[2 * (size_t)nk_ * n + k] & rns::kErrBit) {
+      cudaMemsetAsync(ks_->ops[k]->t.err, 0, sizeof(int), s_);
+      cudaStreamSynchronize(s_);
+      err_ = "a tensor-core product's pipeline wait gave up";
+      return BG_ETIMEOUT;
+    }
     if (h_out_[2 * (size_t)nk_ * n + k] != 0.0) {
       cudaMemsetAsync(ks_->ops[k]->t.err, 0, sizeof(int), s_);
       cudaStreamSynchronize(s_);

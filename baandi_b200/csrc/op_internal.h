@@ -66,6 +66,7 @@ struct bg_op {
   int dens_chunks = 0;  // chunks dens_part holds
   bool vtf_valid = false;  // t.vtf (the FP32 apply's potential) matches t.vt
   bg::TcNl tc;             // tensor-core nonlocal products (BG_PREC_TENSOR)
+  bg::RnsNl rns;           // FP64 nonlocal products on the int8 tensor cores
   // device work arrays of bg_davidson_solve, kept between solves on this operator (the
   // solver takes them in a fixed order and enlarges one only when a solve needs more)
   std::vector<std::unique_ptr<DevBuf>> dv_arena;
@@ -115,15 +116,19 @@ struct bg_kset {
   int* d_errv = nullptr;
   int* h_errv = nullptr;
   bg::TcNl tc;  // tensor-core nonlocal products (BG_PREC_TENSOR)
+  bg::RnsNl rns;  // FP64 nonlocal products on the int8 tensor cores
 };
 
 namespace bg {
 // Launch the local and nonlocal stages of operators [k0, k1) of a set on one stream
 // (cols[k]: the widest block of operator k, used to size the grids).
 // prec: BG_PREC_FP64, BG_PREC_FP32 or BG_PREC_TENSOR (tensor buffers sized beforehand
-// by ensure_nonlocal_tc on tc, or on ks->tc when tc is null).
+// by ensure_nonlocal_tc on tc, or on ks->tc when tc is null).  rns: buffers of the FP64
+// residue products (null: ks->rns).
 int enqueue_range(bg_kset* ks, int k0, int k1, const CallArgs* args, const int64_t* cols, cudaStream_t s,
-                  StageEvents* ev, int prec = 0, TcNl* tc = nullptr);
+                  StageEvents* ev, int prec = 0, TcNl* tc = nullptr, RnsNl* rns = nullptr);
+// Status and message of a device error word read back (0: BG_OK).
+int report_error_bits(bg_ctx* ctx, int bits);
 // Convert the operator's potential to its FP32 copy on stream s if the copy is stale.
 int ensure_potential_float(bg_op* op, cudaStream_t s);
 // Failure message on the context (or the thread's context-free slot) and status.

@@ -1,0 +1,95 @@
+"""FP64 products on the int8 tensor cores (csrc/gemm_rns.cu) against extended-precision sums:
+tile edges, K remainders, every op, split and unsplit A, badly scaled and non-finite input.
+
+Bound of an entry: a row is scaled by a power of two to a 2-norm of 2^57.3 .. 2^58.3 and
+every real part rounded to an integer, so each of its K complex values is off by at most
+2^-1/2 and, by Cauchy-Schwarz, the sum of K products by sqrt(K / 2) (1 / |a| + 1 / |b|) of the
+norms' product in scaled units: sqrt(2 K) 2^-57.3 |a| |b|.  The result is rounded to FP64
+twice more (2^-51 |c| covers that and the final addition).
+"""
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+
+from baandi_b200 import _lib as L
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(1, 1, 1), (64, 16, 3), (127, 15, 64), (128, 16, 65), (129, 17, 63), (255, 128, 130), (257, 129, 1000),
+         (300, 256, 1144), (256, 257, 1146), (513, 40, 1152), (40, 300, 4099)]
+
+
+def product(mode, a, b, c, op, presplit):
+    """a, b, c: CUDA complex128 rows = columns of the column-major matrices."""
+    lib = L.load()
+    m = a.shape[0] if mode == 0 else a.shape[1]
+    k, n = b.shape[1], b.shape[0]
+    rc = lib.bg_test_residue_product(ctypes.c_int32(mode), ctypes.c_int64(m), ctypes.c_int64(n), ctypes.c_int64(k),
+                                     ctypes.c_void_p(a.data_ptr()), ctypes.c_int64(a.shape[1]),
+                                     ctypes.c_void_p(b.data_ptr()), ctypes.c_int64(k),
+                                     ctypes.c_void_p(c.data_ptr()), ctypes.c_int64(m), ctypes.c_int32(op),
+                                     ctypes.c_int32(presplit))
+    assert rc == 0, rc
+
+
+def matrices(mode, m, n, k, seed):
+    rng = np.random.default_rng(seed)
+    z = lambda r, c: rng.standard_normal((r, c)) + 1j * rng.standard_normal((r, c))
+    a = z(m, k) if mode == 0 else z(k, m)
+    return a, z(n, k), z(n, m)
+
+
+def exact(mode, a, b):
+    """(n, m) product in 80-bit arithmetic and the bound's norm products."""
+    left = (a.conj() if mode == 0 else a.T).astype(np.clongdouble)
+    norms = np.linalg.norm(b, axis=1)[:, None] * np.linalg.norm(np.abs(left).astype(np.float64), axis=1)[None, :]
+    return b.astype(np.clongdouble) @ left.T, norms
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("m,n,k", SIZES)
+def test_tile_edges(mode, m, n, k):
+    torch = pytest.importorskip("torch")
+    op, presplit = (m + n + k) % 3, (m + k) % 2
+    a, b, c0 = matrices(mode, m, n, k, m + 7 * n + 31 * k)
+    a[..., 0] *= 1e-3  # a graded row or column
+    c = torch.from_numpy(c0.copy()).cuda()
+    product(mode, torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), c, op, presplit)
+    want, norms = exact(mode, a, b)
+    if op == 1:
+        want = c0 + want
+    if op == 2:
+        want = c0 - want
+    diff = np.abs((c.cpu().numpy() - want).astype(np.complex128))
+    bound = np.sqrt(2 * k) * 2.0 ** -57.3 * norms + 2.0 ** -51 * (np.abs(want).astype(np.float64) + (np.abs(c0) if op else 0.0))
+    assert np.all(diff <= bound), float(np.max(diff / bound))
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_scales_and_nonfinite(mode):
+    torch = pytest.importorskip("torch")
+    m, n, k = 130, 33, 200
+    a, b, c0 = matrices(mode, m, n, k, 5)
+    rows = a if mode == 0 else a.T          # row i of the left factor
+    rows[2] = 0.0
+    b[1] = 0.0
+    want, norms = exact(mode, a, b)
+    ea, eb = np.zeros(m, np.int64), np.zeros(n, np.int64)
+    ea[0], ea[1], eb[0] = 660, -660, -660   # squares overflow and underflow; one product vanishes
+    rows *= np.ldexp(1.0, ea)[:, None]
+    b *= np.ldexp(1.0, eb)[:, None]
+    rows[5, 11] = np.inf
+    b[3, 7] = np.nan
+    c = torch.from_numpy(c0.copy()).cuda()
+    product(mode, torch.from_numpy(np.ascontiguousarray(a)).cuda(), torch.from_numpy(b).cuda(), c, 0, 0)
+    got = c.cpu().numpy()
+    assert np.all(np.isnan(got[3].real)) and np.all(np.isnan(got[:, 5].real))
+    fine = np.ix_(np.arange(n) != 3, np.arange(m) != 5)
+    e = (eb[:, None] + ea[None, :])[fine]
+    w = want[fine].astype(np.complex128)
+    w = np.ldexp(w.real, e) + 1j * np.ldexp(w.imag, e)
+    bound = np.ldexp(np.sqrt(2 * k) * 2.0 ** -57.3 * norms[fine], e) + 2.0 ** -51 * np.abs(w) + 4 * np.finfo(np.float64).smallest_subnormal
+    assert np.all(np.abs(got[fine] - w) <= bound)
