@@ -820,7 +820,9 @@ __global__ void __launch_bounds__(kT) k_w_tri_gs(const Bufs<D>* __restrict__ buf
 // Y[:, c] = H_0 H_1 ... H_{m-3} (s . Z[:, order[c]]) for c < m: kBackCols columns per
 // block, one warp per column; each reflector is staged once per block in shared memory
 // (double-buffered, one barrier per reflector) and applied by every warp to its column.
-constexpr int kBackCols = 6;  // (6 + 2) x 1536 x 16 bytes of shared memory at the largest capacity
+// 7: the 960 columns of the Si216 problem are 138 blocks, one wave of the 148 SMs (a block takes
+// most of an SM's shared memory); 6 columns made 160 blocks run two waves, 2.0 ms a call.
+constexpr int kBackCols = 7;  // (7 + 2) x 1152 x 16 bytes of shared memory at the largest capacity
 template <class D>
 __global__ void __launch_bounds__(kT) k_w_back(const Bufs<D>* __restrict__ bufs, const Ctl* __restrict__ ctl, int cap) {
   using X = Cx<D>;
