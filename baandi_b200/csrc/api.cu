@@ -16,6 +16,7 @@
 #include "gemm_rns.cuh"
 #include "gemm_tc.cuh"
 #include "op_internal.h"
+#include "plane_passes.cuh"
 
 namespace bg {
 static thread_local std::string g_error;
@@ -369,6 +370,7 @@ int build_op(bg_ctx* ctx, const bg_basis_desc* b, const bg_projectors* pr, int64
   T.nxact = (int)xact.size();
   T.yper = plane_lines_per_warp(n0, n1, T.nxact);
   T.yper16 = plane_lines_per_warp(n0, n1, T.nxact, 16);
+  if (plane_any_supported(G)) plane_lines_any(G, T.nxact, &T.yany, &G.xper, &G.dper);
   int rc;
   int* d_int;
   if ((rc = upload(op.get(), grp_stick.data(), grp_stick.size(), &d_int))) return rc;
@@ -578,6 +580,13 @@ int ensure_buf(bg_op* op, double** p, size_t doubles) {
   if (rc) return rc;
   *p = static_cast<double*>(vp);
   return BG_OK;
+}
+
+// Units of a band density whose slices are formed before they are summed: all of them while
+// they fit in 1 GiB.
+int density_group(int units, int nk, const BoxGeo& g) {
+  const double slice = 8.0 * g.n0 * g.n1 * g.n2 * nk;
+  return (int)std::max(1.0, std::min((double)units, std::floor(1073741824.0 / slice)));
 }
 
 size_t grid_points(const bg_op* op) { return (size_t)op->dims[0] * op->dims[1] * op->dims[2]; }
@@ -927,16 +936,9 @@ int bg_op_band_density_sum(bg_op* op, const double* x, int64_t rows, int64_t col
     }
   } else {
     const int units = op->gamma ? (int)((cols + 1) / 2) : (int)cols;
-    // Enough (plane, chunk) blocks for two waves of 148 SMs; chunks sum in order.
-    const int max_chunks = std::max<int>(1, std::min<int64_t>(op->cap_units, (2 * 148 + op->dims[2] - 1) / op->dims[2]));
-    if (!op->dens_part) {
-      if ((rc = ensure_buf(op, &op->dens_part, (size_t)max_chunks * pts))) return rc;
-      op->dens_chunks = max_chunks;
-    }
+    const int group = density_group((int)op->cap_units, 1, op->g);  // the buffer's size, for any block
+    if ((rc = ensure_buf(op, &op->dens_part, (size_t)group * pts))) return rc;
     if ((rc = ensure_buf(op, &op->dens_w, (size_t)op->cap))) return rc;
-    const int want = std::min(units, op->dens_chunks);
-    const int per_chunk = (units + want - 1) / want;
-    const int chunks = (units + per_chunk - 1) / per_chunk;
     const size_t dpc = op->gamma ? (size_t)rows : (size_t)2 * rows;
     const double* dx = x;
     if (ptr_kind == BG_PTR_HOST) {
@@ -954,11 +956,9 @@ int bg_op_band_density_sum(bg_op* op, const double* x, int64_t rows, int64_t col
     a.ldx = a.ldy = (int64_t)dpc;
     a.cols = (int)cols;
     a.units = units;
-    op->launches += launch_density(op->d_tabs, op->gamma ? 1 : 0, op->t.ngroups, op->g, bt, op->dens_w, 0, per_chunk,
-                                   chunks, op->dens_part, op->stream);
     if ((rc = ensure_buf(op, &op->dens_ksum, pts))) return rc;
-    launch_density_reduce(op->dens_part, 1, chunks, op->g, volume, accumulate, op->dens_ksum, dd, op->stream);
-    op->launches += 2;
+    op->launches += launch_density(op->d_tabs, op->gamma ? 1 : 0, op->t.ngroups, op->g, bt, op->dens_w, 0, group, volume,
+                                   accumulate, op->dens_part, op->dens_ksum, dd, op->stream);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
   }
@@ -1197,13 +1197,7 @@ int bg_kset_band_density_sum(bg_kset* ks, const double* const* x, int64_t cols, 
     return BG_OK;
   }
   const int units = ks->gamma ? (int)((cols + 1) / 2) : (int)cols;
-  // one unit per (plane, chunk, k) block while the partial slices fit in 1 GiB (the plane
-  // kernel then carries nothing across units and runs four blocks per SM); otherwise
-  // enough blocks for two waves of 148 SMs.  Chunks sum in order.
-  const bool one = (double)n * units * pts * sizeof(double) <= 1073741824.0;
-  const int want = one ? units : std::max(1, std::min(units, (2 * 148 + g.n2 * n - 1) / (g.n2 * n)));
-  const int per_chunk = (units + want - 1) / want;
-  const int chunks = (units + per_chunk - 1) / per_chunk;
+  const int group = density_group(units, n, g);
   auto grow = [&](double** p, size_t* have, size_t need) -> int {
     if (*have >= need) return BG_OK;
     cudaFree(*p);
@@ -1217,7 +1211,7 @@ int bg_kset_band_density_sum(bg_kset* ks, const double* const* x, int64_t cols, 
     return BG_OK;
   };
   int rc;
-  if ((rc = grow(&ks->dens_part, &ks->dens_part_doubles, (size_t)n * chunks * pts))) return rc;
+  if ((rc = grow(&ks->dens_part, &ks->dens_part_doubles, (size_t)n * group * pts))) return rc;
   if ((rc = grow(&ks->dens_w, &ks->dens_w_doubles, (size_t)n * cols))) return rc;
   if ((rc = grow(&ks->dens_ksum, &ks->dens_ksum_doubles, (size_t)n * pts))) return rc;
   e = cudaMemcpyAsync(ks->dens_w, weights, (size_t)n * cols * sizeof(double), cudaMemcpyHostToDevice, ks->stream);
@@ -1234,10 +1228,8 @@ int bg_kset_band_density_sum(bg_kset* ks, const double* const* x, int64_t cols, 
     a.cols = (int)cols;
     a.units = units;
   }
-  ks->launches += launch_density(ks->d_tabs, ks->gamma, ks->max_groups, g, bt, ks->dens_w, (int)cols, per_chunk,
-                                 chunks, ks->dens_part, ks->stream);
-  launch_density_reduce(ks->dens_part, n, chunks, g, volume, accumulate, ks->dens_ksum, density, ks->stream);
-  ks->launches += 2;
+  ks->launches += launch_density(ks->d_tabs, ks->gamma, ks->max_groups, g, bt, ks->dens_w, (int)cols, group, volume,
+                                 accumulate, ks->dens_part, ks->dens_ksum, density, ks->stream);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
   return BG_OK;
 }

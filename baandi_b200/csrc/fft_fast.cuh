@@ -37,6 +37,28 @@ BG_PLAN(54, 6, 9)
 BG_PLAN(60, 12, 5)
 BG_PLAN(72, 8, 9)
 BG_PLAN(108, 12, 9)
+// lengths of the any-length passes only (fft_any.cuh)
+BG_PLAN(15, 3, 5)
+BG_PLAN(16, 4, 4)
+BG_PLAN(18, 3, 6)
+BG_PLAN(20, 4, 5)
+BG_PLAN(24, 4, 6)
+BG_PLAN(27, 3, 9)
+BG_PLAN(30, 5, 6)
+BG_PLAN(32, 4, 8)
+BG_PLAN(36, 6, 6)
+BG_PLAN(40, 5, 8)
+BG_PLAN(48, 6, 8)
+BG_PLAN(50, 10, 5)
+BG_PLAN(64, 8, 8)
+BG_PLAN(75, 15, 5)
+BG_PLAN(80, 10, 8)
+BG_PLAN(81, 9, 9)
+BG_PLAN(90, 10, 9)
+BG_PLAN(96, 12, 8)
+BG_PLAN(100, 10, 10)
+BG_PLAN(120, 12, 10)
+BG_PLAN(128, 16, 8)
 #undef BG_PLAN
 
 // --------------------------------------------------------------------- butterflies
@@ -171,6 +193,27 @@ struct Dft<9, SIGN, C> {
     }
   }
 };
+// 10 = 5 x 2: a = DFT5(evens), b = DFT5(odds); X[u] = a[u] + w10^u b[u], X[u+5] = a[u] - w10^u b[u].
+template <int SIGN, class C>
+struct Dft<10, SIGN, C> {
+  __device__ __forceinline__ static void run(C* v) {
+    using T = RealOf<C>;
+    C a[5] = {v[0], v[2], v[4], v[6], v[8]}, b[5] = {v[1], v[3], v[5], v[7], v[9]};
+    Dft<5, SIGN, C>::run(a);
+    Dft<5, SIGN, C>::run(b);
+    const T c1 = T(0.8090169943749475), s1 = T(0.5877852522924731);   // 2 pi/10
+    const T c2 = T(0.30901699437494745), s2 = T(0.9510565162951535);  // 4 pi/10
+    b[1] = w_mul<SIGN>(b[1], c1, s1);
+    b[2] = w_mul<SIGN>(b[2], c2, s2);
+    b[3] = w_mul<SIGN>(b[3], -c2, s2);
+    b[4] = w_mul<SIGN>(b[4], -c1, s1);
+#pragma unroll
+    for (int u = 0; u < 5; ++u) {
+      v[u] = cadd(a[u], b[u]);
+      v[u + 5] = csub(a[u], b[u]);
+    }
+  }
+};
 
 // 12 = 3 x 4: a_m = DFT4(v_m, v_{m+3}, v_{m+6}, v_{m+9}); b_m[k1] = a_m[k1] w12^(m k1);
 // X[k1 + 4 k2] = DFT3 over m of b_m[k1].
@@ -200,6 +243,75 @@ struct Dft<12, SIGN, C> {
   }
 };
 
+// 15 = 3 x 5: a_m = DFT5(v_m, v_{m+3}, ...); b_m[k1] = a_m[k1] w15^(m k1); X[k1 + 5 k2] = DFT3
+// over m of b_m[k1].
+template <int SIGN, class C>
+struct Dft<15, SIGN, C> {
+  __device__ __forceinline__ static void run(C* v) {
+    using T = RealOf<C>;
+    C a0[5] = {v[0], v[3], v[6], v[9], v[12]}, a1[5] = {v[1], v[4], v[7], v[10], v[13]},
+      a2[5] = {v[2], v[5], v[8], v[11], v[14]};
+    Dft<5, SIGN, C>::run(a0);
+    Dft<5, SIGN, C>::run(a1);
+    Dft<5, SIGN, C>::run(a2);
+    const T c1 = T(0.9135454576426009), s1 = T(0.4067366430758002);    // 2 pi/15
+    const T c2 = T(0.6691306063588582), s2 = T(0.7431448254773942);    // 4 pi/15
+    const T c3 = T(0.30901699437494745), s3 = T(0.9510565162951535);   // 6 pi/15
+    const T c4 = T(-0.10452846326765347), s4 = T(0.9945218953682733);  // 8 pi/15
+    const T c6 = T(-0.8090169943749475), s6 = T(0.5877852522924731);   // 12 pi/15
+    const T c8 = T(-0.9781476007338057), s8 = T(-0.20791169081775934); // 16 pi/15
+    a1[1] = w_mul<SIGN>(a1[1], c1, s1);
+    a1[2] = w_mul<SIGN>(a1[2], c2, s2);
+    a1[3] = w_mul<SIGN>(a1[3], c3, s3);
+    a1[4] = w_mul<SIGN>(a1[4], c4, s4);
+    a2[1] = w_mul<SIGN>(a2[1], c2, s2);
+    a2[2] = w_mul<SIGN>(a2[2], c4, s4);
+    a2[3] = w_mul<SIGN>(a2[3], c6, s6);
+    a2[4] = w_mul<SIGN>(a2[4], c8, s8);
+#pragma unroll
+    for (int k1 = 0; k1 < 5; ++k1) {
+      C t[3] = {a0[k1], a1[k1], a2[k1]};
+      Dft<3, SIGN, C>::run(t);
+      v[k1] = t[0];
+      v[k1 + 5] = t[1];
+      v[k1 + 10] = t[2];
+    }
+  }
+};
+
+// 16 = 4 x 4: a_m = DFT4(v_m, v_{m+4}, v_{m+8}, v_{m+12}); b_m[k1] = a_m[k1] w16^(m k1);
+// X[k1 + 4 k2] = DFT4 over m of b_m[k1].
+template <int SIGN, class C>
+struct Dft<16, SIGN, C> {
+  __device__ __forceinline__ static void run(C* v) {
+    using T = RealOf<C>;
+    C a[4][4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+#pragma unroll
+      for (int t = 0; t < 4; ++t) a[m][t] = v[m + 4 * t];
+      Dft<4, SIGN, C>::run(a[m]);
+    }
+    const T r = T(0.7071067811865476), c1 = T(0.9238795325112867), s1 = T(0.3826834323650898);  // 2 pi/16
+    a[1][1] = w_mul<SIGN>(a[1][1], c1, s1);
+    a[1][2] = w_mul<SIGN>(a[1][2], r, r);
+    a[1][3] = w_mul<SIGN>(a[1][3], s1, c1);
+    a[2][1] = w_mul<SIGN>(a[2][1], r, r);
+    a[2][2] = irot<SIGN>(a[2][2]);
+    a[2][3] = w_mul<SIGN>(a[2][3], -r, r);
+    a[3][1] = w_mul<SIGN>(a[3][1], s1, c1);
+    a[3][2] = w_mul<SIGN>(a[3][2], -r, r);
+    a[3][3] = w_mul<SIGN>(a[3][3], -c1, -s1);  // w16^9
+#pragma unroll
+    for (int k1 = 0; k1 < 4; ++k1) {
+      C t[4] = {a[0][k1], a[1][k1], a[2][k1], a[3][k1]};
+      Dft<4, SIGN, C>::run(t);
+#pragma unroll
+      for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = t[k2];
+    }
+  }
+};
+
 // --------------------------------------------------------------------- stages
 // Lane index read with a volatile instruction: the per-lane butterfly indices of a stage
 // are then recomputed where the stage runs instead of being hoisted out of an enclosing
@@ -223,11 +335,12 @@ struct StageIo {
   const int* tab = nullptr;
   C* row = nullptr;
   const unsigned* xb = nullptr;  // element bits (4 words, N <= 128)
+  int es = 1;                    // element stride of the passes with ES = 0
 };
 
 __device__ __forceinline__ unsigned xbit(const unsigned* xb, int e) { return (__ldg(xb + (e >> 5)) >> (e & 31)) & 1u; }
 
-// Stage (R, NS) on lines first .. first+count-1 of this warp; ES = element stride.
+// Stage (R, NS) on lines first .. first+count-1 of this warp; ES = element stride (0: io.es).
 // A lane's butterfly index j, its twiddle and its element masks are the same in every
 // round, so they are set up once before the rounds.
 template <int N, int R, int NS, int SIGN, int ES, int IO = 0, class Off, class C>
@@ -237,6 +350,7 @@ __device__ __forceinline__ void stage(C* base, int first, int count, Off off, co
   constexpr int STEP = N / (NS * R);
   constexpr int K = (SPAN + 31) / 32;                 // butterflies per lane when a line exceeds a warp
   constexpr int LPR = SPAN <= 32 ? 32 / SPAN : 1;     // whole lines per round
+  const int es = ES > 0 ? ES : io.es;
   lane = lane_id();
   int jj[K], li[K], oo[K];
   unsigned tin[K], tout[K];
@@ -279,7 +393,7 @@ __device__ __forceinline__ void stage(C* base, int first, int count, Off off, co
         } else {
 #pragma unroll
           for (int t = 0; t < R; ++t)
-            v[q][t] = ((IO & kInMask) == 0 || ((tin[q] >> t) & 1u)) ? base[lo[q] + (jj[q] + t * SPAN) * ES]
+            v[q][t] = ((IO & kInMask) == 0 || ((tin[q] >> t) & 1u)) ? base[lo[q] + (jj[q] + t * SPAN) * es]
                                                                    : mkc<C>(0.0, 0.0);
         }
       }
@@ -310,7 +424,7 @@ __device__ __forceinline__ void stage(C* base, int first, int count, Off off, co
         } else {
 #pragma unroll
           for (int u = 0; u < R; ++u)
-            if ((IO & kOutMask) == 0 || ((tout[q] >> u) & 1u)) base[lo[q] + (oo[q] + u * NS) * ES] = v[q][u];
+            if ((IO & kOutMask) == 0 || ((tout[q] >> u) & 1u)) base[lo[q] + (oo[q] + u * NS) * es] = v[q][u];
         }
       }
     }
@@ -355,6 +469,7 @@ __device__ __forceinline__ void inverse_weight_forward(C* base, int first, int c
   constexpr int SPAN = N / R2;  // == R1
   static_assert(SPAN <= 32, "one butterfly per lane");
   constexpr int LPR = 32 / SPAN;
+  const int es = ES > 0 ? ES : io.es;
   lane = lane_id();
   const int li = lane / SPAN;
   const int j = lane - li * SPAN;
@@ -367,7 +482,7 @@ __device__ __forceinline__ void inverse_weight_forward(C* base, int first, int c
     const int lo = act ? off(line) : 0;
     if (act) {
 #pragma unroll
-      for (int t = 0; t < R2; ++t) v[t] = base[lo + (j + t * SPAN) * ES];
+      for (int t = 0; t < R2; ++t) v[t] = base[lo + (j + t * SPAN) * es];
     }
     __syncwarp();
     if (act) {
@@ -388,7 +503,7 @@ __device__ __forceinline__ void inverse_weight_forward(C* base, int first, int c
       }
       Dft<R2, -1, C>::run(v);
 #pragma unroll
-      for (int u = 0; u < R2; ++u) base[lo + (j * R2 + u) * ES] = v[u];
+      for (int u = 0; u < R2; ++u) base[lo + (j * R2 + u) * es] = v[u];
     }
     __syncwarp();
   }

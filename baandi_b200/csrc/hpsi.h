@@ -21,6 +21,7 @@ struct OpTables {
   int nxact;      // x rows of the plane holding at least one stick
   int yper;       // x rows per warp in the 8-warp plane kernels' y passes
   int yper16;     // the same for the 16-warp plane kernels (one block per SM)
+  int yany;       // the same for the any-length plane kernels (planes_any.cu)
   const int* grp_stick;   // ngroups+1: first stick of each group
   const int* grp_entry;   // ngroups+1: entry range of each group
   const int2* entries;    // complex: (row g, pos); Gamma: (code, pos), code 0 for G=0,
@@ -46,6 +47,7 @@ struct BoxGeo {
   int sg;      // max sticks per group
   int vstride; // doubles between z planes of the transposed potential (even: 16-byte aligned planes)
   int vstridef; // floats between z planes of the FP32 potential (multiple of 4: 16-byte aligned planes)
+  int xper, dper;  // columns per warp of the any-length x passes (apply, density)
   double inv_n;
   FftPlan p0, p1, p2;
   const double2* tw0;  // exp(+2 pi i q/n0), q < n0
@@ -182,17 +184,15 @@ bool ensure_nonlocal_rns(RnsNl* r, int nk, int nproj, int64_t max_cols, int max_
 int launch_nonlocal_rns(const NlDev* nl, const NlShape& sh, int max_rows, int max_cols, const Batch& b, RnsNl* r,
                         int* err, cudaStream_t s, StageEvents* ev);
 
-// Band densities of the blocks of a batch (k = 0 .. b.nk - 1, operator tables tabs[k]
-// and their stick buffers): part[k][c][z][y n0 + x] = sum over the units of chunk c of
-// block k (in unit order) of w |psi(r)|^2, psi the unscaled inverse transform (Gamma:
-// w_a Re^2 + w_b Im^2 of a column pair).  weights: device array, block k's column
-// weights at k wstride; `chunks` chunks of `per_chunk` units per block.
+// out (= or +=) sum over the blocks of a batch (k = 0 .. b.nk - 1, operator tables tabs[k] and
+// their stick buffers) and their units, in order, of w |psi(r)|^2 / volume, psi the unscaled
+// inverse transform (Gamma: w_a Re^2 + w_b Im^2 of a column pair).  weights: device array,
+// block k's column weights at k wstride.  Units pass in groups of `group`: part holds the
+// group's slices, [k][unit of the group][z][y n0 + x]; ksum: scratch of nk grids.  Returns
+// the number of launches.
 int launch_density(const OpTables* tabs, int gamma, int max_groups, const BoxGeo& g, const Batch& b,
-                   const double* weights, int wstride, int per_chunk, int chunks, double* part, cudaStream_t s);
-// out (= or +=) the per-k chunk sums of part / volume, k points in order; ksum: scratch of
-// nk grids (the per-k sums).
-void launch_density_reduce(const double* part, int nk, int chunks, const BoxGeo& g, double volume, int accumulate,
-                           double* ksum, double* out, cudaStream_t s);
+                   const double* weights, int wstride, int group, double volume, int accumulate, double* part,
+                   double* ksum, double* out, cudaStream_t s);
 // out[i] = *err[i], then *err[i] = 0 (the operators' error words, read and cleared).
 void launch_gather_errors(int* const* err, int n, int* out, cudaStream_t s);
 // Copy n doubles from src to each of the ndst device pointers in dst (a device array).

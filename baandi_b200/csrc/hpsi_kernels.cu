@@ -22,7 +22,8 @@
 #include "hpsi.h"
 #include "gemm_rns.cuh"
 #include "gemm_tc.cuh"
-#include "fft_fast.cuh"
+#include "fft_any.cuh"
+#include "plane_passes.cuh"
 #include "gemm_tiles.cuh"
 
 #include <algorithm>
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(N == 0 ? 256 : 128, sticks_blocks_per_sm<N, C>
   }
   if (bad) atomicOr(t.err, 1);
   if constexpr (N == 0) {
-    fft_lines<1>(st, cnt, LineOffStride{g.ld2}, 1, g.p2, tw);
+    fft_block_lines<1>(st, cnt, g.ld2, g.p2, tw);
   } else {
     __syncthreads();
     fast::pass<N, 1, 1>(st, cnt, LineOffStride{fast::pitch_of<N>()}, tw);
@@ -159,6 +160,7 @@ __global__ void __launch_bounds__(N == 0 ? 256 : 128, sticks_blocks_per_sm<N, C>
 }
 
 // ---------------------------------------------------------------- pass 2
+// Planes with an axis outside fft_any.cuh (shorter than 15, or 125): runtime radices.
 __global__ void __launch_bounds__(512) k_planes(const OpTables* __restrict__ tabs, BoxGeo g, Batch b) {
   const OpTables& t = tabs[blockIdx.z];
   const CallArgs a = resolve(b.a[blockIdx.z]);
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(N == 0 ? 256 : 128, sticks_blocks_per_sm<N, C>
   tiles::async_wait<0>();
   __syncthreads();
   if constexpr (N == 0) {
-    fft_lines<-1>(st, cnt, LineOffStride{g.ld2}, 1, g.p2, tw);
+    fft_block_lines<-1>(st, cnt, g.ld2, g.p2, tw);
   } else {
     fast::pass<N, -1, 1>(st, cnt, LineOffStride{fast::pitch_of<N>()}, tw);
   }
@@ -513,37 +515,19 @@ __global__ void __launch_bounds__(256, 2) k_back(const NlDev* __restrict__ nls, 
 // Reference: crates/dft-physics/src/distributed_complex.rs:485-547 (complex, sum in
 // band order of weight |u(r)|^2 / volume), distributed_real_gamma.rs:744-785 (Gamma
 // pairs: weight_a Re^2 + weight_b Im^2).
-__device__ __forceinline__ void density_weights(const CallArgs& a, int gamma, const double* __restrict__ w, int unit,
-                                                double* wa, double* wb) {
-  if (gamma) {
-    *wa = w[2 * unit];
-    *wb = 2 * unit + 1 < a.cols ? w[2 * unit + 1] : 0.0;
-  } else {
-    *wa = *wb = w[unit];
-  }
-}
-
-// Blocks of k_density_planes_fast per SM: 2 up to 45^3 planes (128 registers), 1 above,
-// where the loop over units keeps more stage indices live than 128 registers hold.
+// Tuned cubic lengths, one unit per (z plane, unit of the group, k point) block: the y inverse
+// on the x rows holding sticks (first stage straight from the stick row), the x inverse on
+// every column y (rows without sticks are zero and not loaded), then w |psi|^2 to the block's
+// own slice.  Blocks as k_planes_fast's: 64 registers up to 72^3, sixteen warps at 108^3.  (A
+// block looping over units and adding into its slice held every stage's indices, 255 registers
+// and one block of eight warps: 11.0 ms for the 480 Si216 bands.)
 template <int N>
-constexpr int density_blocks_per_sm() {
-  return N <= 45 ? 2 : 1;
-}
-
-// One block per (z plane, chunk of units, k point).  Per unit: the y inverse on the x
-// rows holding sticks (first stage straight from the stick row), the x inverse on every
-// column y (rows without sticks are zero and not loaded), then w |psi|^2 added point by
-// point.  Up to 4 points per thread the sums stay in registers and the block writes its
-// slice once; larger planes add into the slice in global memory unit by unit.
-template <int N, bool ONE = false>
-__global__ void __launch_bounds__(256, ONE ? 4 : density_blocks_per_sm<N>()) k_density_planes_fast(
-    const OpTables* __restrict__ tabs, BoxGeo g, Batch b, int gamma, const double* __restrict__ w, int wstride,
-    int per_chunk, double* __restrict__ part) {
+__global__ void __launch_bounds__(planes_threads<N, double2>(), planes_threads<N, double2>() == 512 ? 1 : 4)
+    k_density_planes_fast(const OpTables* __restrict__ tabs, BoxGeo g, Batch b, int gamma, const double* __restrict__ w,
+                          int wstride, int unit0, double* __restrict__ part) {
   using Pl = fast::Plan<N>;
   static_assert(Pl::nst == 2, "two-stage plans");
   constexpr int R1 = Pl::radix[0], R2 = Pl::radix[1];
-  constexpr int QP = (N * N + 255) / 256;
-  constexpr bool REG = !ONE && QP <= 4;
   const OpTables& t = tabs[blockIdx.z];
   const CallArgs& a = b.a[blockIdx.z];
   w += (int64_t)blockIdx.z * wstride;
@@ -557,28 +541,25 @@ __global__ void __launch_bounds__(256, ONE ? 4 : density_blocks_per_sm<N>()) k_d
   for (int i = threadIdx.x; i < N; i += blockDim.x) tw[i] = g.tw0[i];
   for (int i = threadIdx.x; i < nx; i += blockDim.x) rows[i] = t.xact[i] * P;
   double* acc = part + ((int64_t)chunk * N + z) * (N * N);
-  const int u0 = blockIdx.y * per_chunk, u1 = min(a.units, u0 + per_chunk);
-  double racc[REG ? QP : 1];
-#pragma unroll
-  for (int q = 0; q < (REG ? QP : 1); ++q) racc[q] = 0.0;
-  if (u0 >= u1 && !REG)  // a k point with fewer units than the widest: its chunk adds nothing
+  const int unit = unit0 + blockIdx.y;
+  if (unit >= a.units) {  // a k point with fewer units than the widest adds nothing
     for (int i = threadIdx.x; i < N * N; i += blockDim.x) acc[i] = 0.0;
-  __syncthreads();
-  fast::StageIo<double2> io;
-  io.tab = t.line_stick;
-  io.xb = t.xbits;
-  const int lane = threadIdx.x & 31;
-  // ONE (one unit per block): no state is carried across units
-  for (int unit = u0; unit < (ONE ? min(u1, u0 + 1) : u1); ++unit) {
+  } else {
+    __syncthreads();
+    fast::StageIo<double2> io;
+    io.tab = t.line_stick;
+    io.xb = t.xbits;
     io.row = t.sbuf + ((int64_t)unit * N + z) * t.S;
+    const int lane = threadIdx.x & 31;
+    constexpr int kWarps = planes_threads<N, double2>() / 32;
     int first, count;
-    fast::owned_block(nx, t.yper, &first, &count);
+    fast::owned_block(nx, kWarps == 16 ? t.yper16 : t.yper, &first, &count);
     if (count > 0) {
       fast::stage<N, R1, 1, 1, 1, fast::kInGlobal>(pl, first, count, LineOffTable{rows}, tw, lane, io);
       fast::stage<N, R2, R1, 1, 1>(pl, first, count, LineOffTable{rows}, tw, lane);
     }
     __syncthreads();
-    constexpr int xper = fast::balanced_lines<N, 1, 1>(N, 8);
+    constexpr int xper = fast::balanced_lines<N, 1, 1>(N, kWarps);
     fast::owned_block(N, xper, &first, &count);
     if (count > 0) {
       fast::stage<N, R1, 1, 1, P, fast::kInMask>(pl, first, count, LineOffCols{}, tw, lane, io);
@@ -587,88 +568,64 @@ __global__ void __launch_bounds__(256, ONE ? 4 : density_blocks_per_sm<N>()) k_d
     __syncthreads();
     double wa, wb;
     density_weights(a, gamma, w, unit, &wa, &wb);
-    if constexpr (REG) {
-#pragma unroll
-      for (int q = 0; q < QP; ++q) {
-        const int i = threadIdx.x + 256 * q;
-        if (i < N * N) {
-          const int y = i / N, x = i - y * N;
-          const double2 p = pl[x * P + y];
-          racc[q] += wa * (p.x * p.x);
-          racc[q] += wb * (p.y * p.y);
-        }
-      }
-    } else {
-      for (int i = threadIdx.x; i < N * N; i += blockDim.x) {
-        const int y = i / N, x = i - y * N;
-        const double2 p = pl[x * P + y];
-        double d = unit == u0 ? 0.0 : acc[i];
-        d += wa * (p.x * p.x);
-        d += wb * (p.y * p.y);
-        acc[i] = d;
-      }
-    }
-    __syncthreads();
-  }
-  if constexpr (REG) {
-#pragma unroll
-    for (int q = 0; q < QP; ++q) {
-      const int i = threadIdx.x + 256 * q;
-      if (i < N * N) acc[i] = racc[q];
+    for (int i = threadIdx.x; i < N * N; i += blockDim.x) {
+      const int y = i / N, x = i - y * N;
+      const double2 p = pl[x * P + y];
+      double d = wa * (p.x * p.x);
+      d += wb * (p.y * p.y);
+      acc[i] = d;
     }
   }
 }
 
+// The same for planes outside fft_any.cuh.
 __global__ void __launch_bounds__(256, 1) k_density_planes(const OpTables* __restrict__ tabs, BoxGeo g, Batch b,
                                                         int gamma, const double* __restrict__ w, int wstride,
-                                                        int per_chunk, double* __restrict__ part) {
+                                                        int unit0, double* __restrict__ part) {
   const OpTables& t = tabs[blockIdx.z];
   const CallArgs& a = b.a[blockIdx.z];
-  w += (int64_t)blockIdx.z * wstride;
-  const int z = blockIdx.x, chunk = blockIdx.y + blockIdx.z * gridDim.y;
-  const int u0 = blockIdx.y * per_chunk, u1 = min(a.units, u0 + per_chunk);
+  const int z = blockIdx.x, unit = unit0 + blockIdx.y;
   extern __shared__ double2 sm[];
   double2* tw0 = sm;
   double2* tw1 = tw0 + g.n0;
   double2* pl = tw1 + g.n1;
+  const int np = g.n0 * g.pitch, pts = g.n0 * g.n1;
+  double* acc = part + ((int64_t)(blockIdx.y + blockIdx.z * gridDim.y) * g.n2 + z) * pts;
+  if (unit >= a.units) {
+    for (int i = threadIdx.x; i < pts; i += blockDim.x) acc[i] = 0.0;
+    return;
+  }
   for (int i = threadIdx.x; i < g.n0; i += blockDim.x) tw0[i] = g.tw0[i];
   for (int i = threadIdx.x; i < g.n1; i += blockDim.x) tw1[i] = g.tw1[i];
-  const int np = g.n0 * g.pitch, pts = g.n0 * g.n1;
-  double* acc = part + ((int64_t)chunk * g.n2 + z) * pts;
-  if (u0 >= u1)
-    for (int i = threadIdx.x; i < pts; i += blockDim.x) acc[i] = 0.0;
-  for (int unit = u0; unit < u1; ++unit) {
-    for (int i = threadIdx.x; i < np; i += blockDim.x) pl[i] = make_double2(0.0, 0.0);
-    __syncthreads();
-    const double2* row = t.sbuf + ((int64_t)unit * g.n2 + z) * t.S;
-    for (int s = threadIdx.x; s < t.S; s += blockDim.x) pl[t.stick_plane[s]] = row[s];
-    fft_lines<1>(pl, t.nxact, LineOffRows{t.xact, g.pitch}, 1, g.p1, tw1);
-    fft_lines<1>(pl, g.n1, LineOffCols{}, g.pitch, g.p0, tw0);
-    double wa, wb;
-    density_weights(a, gamma, w, unit, &wa, &wb);
-    for (int i = threadIdx.x; i < pts; i += blockDim.x) {
-      const int y = i / g.n0, x = i - y * g.n0;
-      const double2 p = pl[x * g.pitch + y];
-      double d = unit == u0 ? 0.0 : acc[i];
-      d += wa * (p.x * p.x);
-      d += wb * (p.y * p.y);
-      acc[i] = d;
-    }
-    __syncthreads();
+  for (int i = threadIdx.x; i < np; i += blockDim.x) pl[i] = make_double2(0.0, 0.0);
+  __syncthreads();
+  const double2* row = t.sbuf + ((int64_t)unit * g.n2 + z) * t.S;
+  for (int s = threadIdx.x; s < t.S; s += blockDim.x) pl[t.stick_plane[s]] = row[s];
+  fft_lines<1>(pl, t.nxact, LineOffRows{t.xact, g.pitch}, 1, g.p1, tw1);
+  fft_lines<1>(pl, g.n1, LineOffCols{}, g.pitch, g.p0, tw0);
+  double wa, wb;
+  density_weights(a, gamma, w + (int64_t)blockIdx.z * wstride, unit, &wa, &wb);
+  for (int i = threadIdx.x; i < pts; i += blockDim.x) {
+    const int y = i / g.n0, x = i - y * g.n0;
+    const double2 p = pl[x * g.pitch + y];
+    double d = wa * (p.x * p.x);
+    d += wb * (p.y * p.y);
+    acc[i] = d;
   }
 }
 
-// ksum[k][q] = (sum_c part[k][c][q]) / volume, chunks in order (q in the partial slices'
-// z, y, x order); blockIdx.y = k, so the k points' chains run side by side.
+// ksum[k][q] (first: =, else +=) sum_c part[k][c][q], units in order (q in the partial slices'
+// z, y, x order), divided by the volume after the last group; blockIdx.y = k, so the k points'
+// chains run side by side.
 __global__ void k_density_sum_chunks(const double* __restrict__ part, int chunks, int64_t total, double volume,
-                                     double* __restrict__ ksum) {
+                                     int first, int last, double* __restrict__ ksum) {
   const int k = blockIdx.y;
   const double* pk = part + (int64_t)k * chunks * total;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
-    double s = 0.0;
+    double s = first ? 0.0 : ksum[(int64_t)k * total + q];
 #pragma unroll 8
     for (int c = 0; c < chunks; ++c) s += pk[(int64_t)c * total + q];
-    ksum[(int64_t)k * total + q] = s / volume;
+    ksum[(int64_t)k * total + q] = last ? s / volume : s;
   }
 }
 
@@ -763,15 +720,21 @@ static void local_kernels(const OpTables* tabs, const BoxGeo& g, const Batch& b,
     return;  // the FP32 apply needs a compile-time plan (checked by the callers)
   } else {
     { StageScope sc(ev, 0, s); k_sticks_inverse<GAMMA, N, C><<<sgrid, st, ss, s>>>(tabs, g, b); }
-    if constexpr (N == 0) {
+    {
       StageScope sc(ev, 1, s);
-      k_planes<<<pgrid, 512, ps, s>>>(tabs, g, b);
-    } else {
-      StageScope sc(ev, 1, s);
-      if (g.n0 == N && g.n1 == N)
-        k_planes_fast<N, C><<<pgrid, planes_threads<N, C>(), ps, s>>>(tabs, g, b);
-      else if constexpr (sizeof(C) == sizeof(double2))
-        k_planes<<<pgrid, 512, ps, s>>>(tabs, g, b);
+      bool done = false;
+      if constexpr (N != 0) {
+        if (g.n0 == N && g.n1 == N) {
+          k_planes_fast<N, C><<<pgrid, planes_threads<N, C>(), ps, s>>>(tabs, g, b);
+          done = true;
+        }
+      }
+      if constexpr (sizeof(C) == sizeof(double2)) {
+        if (!done && plane_any_supported(g))
+          launch_planes_any(tabs, g, b, pgrid, s);
+        else if (!done)
+          k_planes<<<pgrid, 512, ps, s>>>(tabs, g, b);
+      }
     }
     { StageScope sc(ev, 2, s); k_sticks_forward<GAMMA, N, C><<<sgrid, st, ss, s>>>(tabs, g, b); }
   }
@@ -837,52 +800,71 @@ size_t density_smem_bytes(const BoxGeo& g) {
   return sizeof(double2) * ((size_t)g.n0 + g.n1 + (size_t)g.n0 * g.pitch) + (fast ? sizeof(int) * (size_t)g.n0 : 0);
 }
 
+// Sticks of every unit (once), then the planes and their sum group by group.
 template <int N>
-static void density_kernels(const OpTables* tabs, int gamma, int max_groups, const BoxGeo& g, const Batch& b,
-                            int max_units, const double* w, int wstride, int per_chunk, int chunks, double* part,
-                            cudaStream_t s) {
+static void density_sticks(const OpTables* tabs, int gamma, const BoxGeo& g, const Batch& b, dim3 sgrid,
+                           cudaStream_t s) {
   constexpr int st = N == 0 ? 256 : 128;
-  const dim3 sgrid(max_groups, max_units, b.nk);
-  const size_t ss = stick_smem_bytes(g), ds = density_smem_bytes(g);
+  const size_t ss = stick_smem_bytes(g);
   if (gamma)
     k_sticks_inverse<true, N><<<sgrid, st, ss, s>>>(tabs, g, b);
   else
     k_sticks_inverse<false, N><<<sgrid, st, ss, s>>>(tabs, g, b);
-  const dim3 dgrid(g.n2, chunks, b.nk);
+}
+
+template <int N>
+static void density_planes(const OpTables* tabs, int gamma, const BoxGeo& g, const Batch& b, const double* w,
+                           int wstride, int unit0, double* part, dim3 dgrid, cudaStream_t s) {
+  const size_t ds = density_smem_bytes(g);
   if constexpr (N != 0) {
     if (g.n0 == N && g.n1 == N) {
-      if (per_chunk == 1)
-        k_density_planes_fast<N, true><<<dgrid, 256, ds, s>>>(tabs, g, b, gamma, w, wstride, per_chunk, part);
-      else
-        k_density_planes_fast<N><<<dgrid, 256, ds, s>>>(tabs, g, b, gamma, w, wstride, per_chunk, part);
+      k_density_planes_fast<N><<<dgrid, planes_threads<N, double2>(), ds, s>>>(tabs, g, b, gamma, w, wstride, unit0,
+                                                                               part);
       return;
     }
   }
-  k_density_planes<<<dgrid, 256, ds, s>>>(tabs, g, b, gamma, w, wstride, per_chunk, part);
+  if (plane_any_supported(g))
+    launch_density_any(tabs, g, b, gamma, w, wstride, unit0, part, dgrid, s);
+  else
+    k_density_planes<<<dgrid, 256, ds, s>>>(tabs, g, b, gamma, w, wstride, unit0, part);
 }
 
 int launch_density(const OpTables* tabs, int gamma, int max_groups, const BoxGeo& g, const Batch& b,
-                   const double* weights, int wstride, int per_chunk, int chunks, double* part, cudaStream_t s) {
+                   const double* weights, int wstride, int group, double volume, int accumulate, double* part,
+                   double* ksum, double* out, cudaStream_t s) {
   int max_units = 0;
   for (int k = 0; k < b.nk; ++k) max_units = max(max_units, b.a[k].units);
   if (max_units == 0 || b.nk == 0) return 0;
-  switch (g.n2) {
-#define BG_DENS(NN) \
-  case NN: density_kernels<NN>(tabs, gamma, max_groups, g, b, max_units, weights, wstride, per_chunk, chunks, part, s); break;
-    BG_DENS(25) BG_DENS(45) BG_DENS(54) BG_DENS(60) BG_DENS(72) BG_DENS(108)
-#undef BG_DENS
-    default: density_kernels<0>(tabs, gamma, max_groups, g, b, max_units, weights, wstride, per_chunk, chunks, part, s); break;
-  }
-  return 2;
-}
-
-void launch_density_reduce(const double* part, int nk, int chunks, const BoxGeo& g, double volume, int accumulate,
-                           double* ksum, double* out, cudaStream_t s) {
   const int64_t total = (int64_t)g.n0 * g.n1 * g.n2;
-  const int bx = (int)std::min<int64_t>((total + 255) / 256, std::max<int64_t>(1, 148 * 8 / std::max(nk, 1) + 1));
-  k_density_sum_chunks<<<dim3(bx, nk), 256, 0, s>>>(part, chunks, total, volume, ksum);
+  const int bx = (int)std::min<int64_t>((total + 255) / 256, std::max<int64_t>(1, 148 * 8 / std::max(b.nk, 1) + 1));
+  const dim3 sgrid(max_groups, max_units, b.nk);
+  int launches = 2;
+#define BG_DENS(CALL)                                                                             \
+  switch (g.n2) {                                                                                 \
+    case 25: CALL(25); break;                                                                     \
+    case 45: CALL(45); break;                                                                     \
+    case 54: CALL(54); break;                                                                     \
+    case 60: CALL(60); break;                                                                     \
+    case 72: CALL(72); break;                                                                     \
+    case 108: CALL(108); break;                                                                   \
+    default: CALL(0); break;                                                                      \
+  }
+#define BG_STICKS(NN) density_sticks<NN>(tabs, gamma, g, b, sgrid, s)
+  BG_DENS(BG_STICKS)
+#undef BG_STICKS
+  for (int u0 = 0; u0 < max_units; u0 += group) {
+    const int n = std::min(group, max_units - u0);
+    const dim3 dgrid(g.n2, n, b.nk);
+#define BG_PLANES(NN) density_planes<NN>(tabs, gamma, g, b, weights, wstride, u0, part, dgrid, s)
+    BG_DENS(BG_PLANES)
+#undef BG_PLANES
+    k_density_sum_chunks<<<dim3(bx, b.nk), 256, 0, s>>>(part, n, total, volume, u0 == 0, u0 + n >= max_units, ksum);
+    launches += 2;
+  }
+#undef BG_DENS
   const int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 8);
-  k_density_sum_k<<<blocks, 256, 0, s>>>(ksum, nk, g.n0, g.n1, g.n2, accumulate, out);
+  k_density_sum_k<<<blocks, 256, 0, s>>>(ksum, b.nk, g.n0, g.n1, g.n2, accumulate, out);
+  return launches;
 }
 
 __global__ void k_gather_errors(int* const* __restrict__ err, int n, int* __restrict__ out) {
@@ -974,8 +956,6 @@ static void configure_one(cudaError_t& e, size_t plane_smem, size_t stick_smem) 
     if constexpr (GAMMA) {
       set((const void*)k_density_planes_fast<N>, plane_smem);
       carve((const void*)k_density_planes_fast<N>);
-      set((const void*)k_density_planes_fast<N, true>, plane_smem);
-      carve((const void*)k_density_planes_fast<N, true>);
     }
   }
 }
@@ -993,7 +973,7 @@ int configure_kernels(size_t plane_smem, size_t stick_smem) {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute((const void*)k_back<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)tiles::nn64m_smem_bytes<double2>());
-  if (e != cudaSuccess) return 1;
+  if (e != cudaSuccess || configure_planes_any()) return 1;
   e = cudaFuncSetAttribute((const void*)k_planes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute((const void*)k_density_planes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem);

@@ -57,13 +57,12 @@ struct bg_op {
   bool is_dense = false;
   double* dense = nullptr;
   // Lazily allocated: a potential change in the layout of t.vt, a C-order grid for
-  // host potentials and densities, band weights, per-chunk density partial sums.
+  // host potentials and densities, band weights, density slices of a group of units.
   double* vchange = nullptr;
   double* grid = nullptr;
   double* dens_w = nullptr;
   double* dens_part = nullptr;
   double* dens_ksum = nullptr;  // one grid: the reduction's per-k sum
-  int dens_chunks = 0;  // chunks dens_part holds
   bool vtf_valid = false;  // t.vtf (the FP32 apply's potential) matches t.vt
   bg::TcNl tc;             // tensor-core nonlocal products (BG_PREC_TENSOR)
   bg::RnsNl rns;           // FP64 nonlocal products on the int8 tensor cores

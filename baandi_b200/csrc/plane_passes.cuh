@@ -1,18 +1,9 @@
-// Shared by the plane kernels of the compile-time lengths (hpsi_kernels.cu) and of the
-// runtime plans (planes_rt.cu).
+// Shared by the plane kernels of the tuned cubic lengths (hpsi_kernels.cu) and of the other
+// lengths (planes_any.cu).
 #pragma once
-#include "fft_rt.cuh"
 #include "hpsi.h"
 
 namespace bg {
-
-struct LineOffTable {
-  const int* off;
-  __device__ __forceinline__ int operator()(int l) const { return off[l]; }
-};
-struct LineOffCols {
-  __device__ __forceinline__ int operator()(int l) const { return l; }
-};
 
 __device__ __forceinline__ void density_weights(const CallArgs& a, int gamma, const double* __restrict__ w, int unit,
                                                 double* wa, double* wb) {
@@ -24,11 +15,19 @@ __device__ __forceinline__ void density_weights(const CallArgs& a, int gamma, co
   }
 }
 
-// Planes of any n0 x n1 (planes_rt.cu): the apply's passes and the band density's.
-void launch_runtime_planes(const OpTables* tabs, const BoxGeo& g, const Batch& b, dim3 grid, size_t smem,
-                           cudaStream_t s);
-void launch_runtime_density(const OpTables* tabs, const BoxGeo& g, const Batch& b, int gamma, const double* w,
-                            int wstride, int per_chunk, double* part, dim3 grid, size_t smem, cudaStream_t s);
-int configure_runtime_planes(size_t plane_smem);
+// Shared memory of a plane block that leaves room for a second one on the SM.
+constexpr size_t kPlaneAnyPair = 113 * 1024;
+
+// The most one block takes: the 227 KB a block may have, less its static part.
+constexpr size_t kPlaneAnyMost = 226 * 1024;
+
+// Whether both axes of the plane have a pass in fft_any.cuh and the plane fits.
+bool plane_any_supported(const BoxGeo& g);
+// x rows and columns per warp of the passes over nlines x rows.
+void plane_lines_any(const BoxGeo& g, int nlines, int* yany, int* xper, int* dper);
+void launch_planes_any(const OpTables* tabs, const BoxGeo& g, const Batch& b, dim3 grid, cudaStream_t s);
+void launch_density_any(const OpTables* tabs, const BoxGeo& g, const Batch& b, int gamma, const double* w, int wstride,
+                        int unit0, double* part, dim3 grid, cudaStream_t s);
+int configure_planes_any();
 
 }  // namespace bg
