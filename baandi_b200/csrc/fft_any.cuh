@@ -4,8 +4,7 @@
 // one kernel, the lengths' address and twiddle work is hoisted together and spills.  Their
 // arguments sit in shared memory (a Pass per block), so a call costs a few instructions.
 //
-// Field grid of 72^3: 12.4 us per axis against 23.4 us with the runtime engine of fft_dev.cuh (16 us
-// of it from the lines' FFTs, the rest from the index arithmetic around them).
+// Field grid of 72^3: 16 us per axis against 23.4 us with the runtime engine of fft_dev.cuh.
 #pragma once
 #include "fft_fast.cuh"
 

@@ -21,6 +21,7 @@
 #include <memory>
 #include <vector>
 
+#include "launch_chain.cuh"
 #include "fft_any.cuh"
 #include "op_internal.h"
 
@@ -78,6 +79,7 @@ __device__ __forceinline__ double block_sum(double v, double* sm) {
 __global__ void __launch_bounds__(kFieldThreads) k_f_xc(const double* __restrict__ rho, int64_t total,
                                                         double* __restrict__ vxc, double2* __restrict__ work,
                                                         double* __restrict__ part, int* err) {
+  chain_wait();
   __shared__ double sm[kFieldThreads];
   double s_ex = 0.0, s_vx = 0.0;
   bool bad = false;
@@ -120,6 +122,7 @@ __device__ __forceinline__ int64_t line_base(const Box3& b, int axis, int64_t L,
 template <int SIGN>
 __global__ void __launch_bounds__(kFieldThreads) k_f_lines(double2* __restrict__ data, Box3 b, int axis, FftPlan plan,
                                                            const double2* __restrict__ twg) {
+  chain_wait();
   extern __shared__ double2 fsm[];
   const int n = b.n[axis];
   const int ld = n | 1;
@@ -165,6 +168,7 @@ struct Recip {
 
 __global__ void __launch_bounds__(kFieldThreads) k_f_poisson(double2* __restrict__ work, Box3 bx, Recip rc,
                                                              double inv_n) {
+  chain_wait();
   for (int64_t p = blockIdx.x * (int64_t)kFieldThreads + threadIdx.x; p < bx.total;
        p += (int64_t)gridDim.x * kFieldThreads) {
     if (p == 0) {
@@ -191,6 +195,7 @@ __global__ void __launch_bounds__(kFieldThreads) k_f_collect(const double2* __re
                                                              const double* __restrict__ vxc, int64_t total,
                                                              double* __restrict__ v_h, double* __restrict__ v_hxc,
                                                              double* __restrict__ part) {
+  chain_wait();
   __shared__ double sm[kFieldThreads];
   double s_eh = 0.0;
   for (int64_t p = blockIdx.x * (int64_t)kFieldThreads + threadIdx.x; p < total;
@@ -208,6 +213,7 @@ __global__ void __launch_bounds__(kFieldThreads) k_f_collect(const double2* __re
 // walking the 592 x 3 sums took 52 us of the 460 us Si64 field step, a chain of dependent loads.)
 __global__ void __launch_bounds__(kFieldThreads) k_f_energies(const double* __restrict__ part, int blocks, double dv,
                                                               double* __restrict__ out) {
+  chain_wait();
   __shared__ double sm[kFieldThreads];
   double s[3] = {0.0, 0.0, 0.0};
   for (int i = threadIdx.x; i < blocks; i += kFieldThreads)
@@ -224,15 +230,18 @@ __global__ void __launch_bounds__(kFieldThreads) k_f_energies(const double* __re
 // 173-237): forward picks FFT(rho)/N on the half-sphere indices; inverse forms
 // 2 Re(sum_half c_G e^{iGr}) - Re c_0 from the half-sphere coefficients alone.
 __global__ void k_f_load_real(const double* __restrict__ rho, int64_t total, double2* __restrict__ work) {
+  chain_wait();
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < total; p += (int64_t)gridDim.x * blockDim.x)
     work[p] = make_double2(rho[p], 0.0);
 }
 __global__ void k_f_zero(double2* __restrict__ work, int64_t total) {
+  chain_wait();
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < total; p += (int64_t)gridDim.x * blockDim.x)
     work[p] = make_double2(0.0, 0.0);
 }
 __global__ void k_f_pick(const double2* __restrict__ work, const int64_t* __restrict__ idx, int64_t n, double inv_n,
                          double2* __restrict__ out) {
+  chain_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const double2 z = work[idx[i]];
     out[i] = make_double2(z.x * inv_n, z.y * inv_n);
@@ -240,6 +249,7 @@ __global__ void k_f_pick(const double2* __restrict__ work, const int64_t* __rest
 }
 __global__ void k_f_place(const double2* __restrict__ c, const int64_t* __restrict__ idx, int64_t n,
                           double2* __restrict__ work, int* err) {
+  chain_wait();
   bool bad = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const double2 z = c[i];
@@ -250,6 +260,7 @@ __global__ void k_f_place(const double2* __restrict__ c, const int64_t* __restri
 }
 __global__ void k_f_half_real(const double2* __restrict__ work, const double2* __restrict__ c, int64_t i0,
                               int64_t total, double* __restrict__ rho) {
+  chain_wait();
   const double g0 = i0 >= 0 ? c[i0].x : 0.0;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < total; p += (int64_t)gridDim.x * blockDim.x)
     rho[p] = 2.0 * work[p].x - g0;
@@ -419,18 +430,18 @@ int bg_fields_lda_hartree(bg_fields* f, const double* density, double* v_hxc, do
     vh = v_h ? f->stage_vh : nullptr;
   }
   const Box3 b = f->box;
-  k_f_xc<<<kFieldBlocks, kFieldThreads, 0, f->stream>>>(rho, total, f->vxc, f->work, f->part, f->err);
+  launch_chained(k_f_xc, kFieldBlocks, kFieldThreads, 0, f->stream, rho, total, f->vxc, f->work, f->part, f->err);
   for (int a = 2; a >= 0; --a) {
     const int blocks = (int)((total / b.n[a] + kLines - 1) / kLines);
-    k_f_lines<-1><<<blocks, kFieldThreads, lines_smem(b.n[a]), f->stream>>>(f->work, b, a, f->plan[a], f->tw[a]);
+    launch_chained(k_f_lines<-1>, blocks, kFieldThreads, lines_smem(b.n[a]), f->stream, f->work, b, a, f->plan[a], f->tw[a]);
   }
-  k_f_poisson<<<kFieldBlocks, kFieldThreads, 0, f->stream>>>(f->work, b, f->rc, 1.0 / (double)total);
+  launch_chained(k_f_poisson, kFieldBlocks, kFieldThreads, 0, f->stream, f->work, b, f->rc, 1.0 / (double)total);
   for (int a = 0; a < 3; ++a) {
     const int blocks = (int)((total / b.n[a] + kLines - 1) / kLines);
-    k_f_lines<1><<<blocks, kFieldThreads, lines_smem(b.n[a]), f->stream>>>(f->work, b, a, f->plan[a], f->tw[a]);
+    launch_chained(k_f_lines<1>, blocks, kFieldThreads, lines_smem(b.n[a]), f->stream, f->work, b, a, f->plan[a], f->tw[a]);
   }
-  k_f_collect<<<kFieldBlocks, kFieldThreads, 0, f->stream>>>(f->work, rho, f->vxc, total, vh, out, f->part);
-  k_f_energies<<<1, kFieldThreads, 0, f->stream>>>(f->part, kFieldBlocks, f->volume / (double)total, f->energies);
+  launch_chained(k_f_collect, kFieldBlocks, kFieldThreads, 0, f->stream, f->work, rho, f->vxc, total, vh, out, f->part);
+  launch_chained(k_f_energies, 1, kFieldThreads, 0, f->stream, f->part, kFieldBlocks, f->volume / (double)total, f->energies);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
   if ((e = cudaMemcpyAsync(f->energies_host, f->energies, sizeof(double) * 3, cudaMemcpyDeviceToHost, f->stream)) !=
           cudaSuccess ||
@@ -484,9 +495,9 @@ static void f_transform(bg_fields* f, int sign) {
     const int a = sign < 0 ? 2 - i : i;
     const int blocks = (int)((b.total / b.n[a] + kLines - 1) / kLines);
     if (sign < 0)
-      k_f_lines<-1><<<blocks, kFieldThreads, lines_smem(b.n[a]), f->stream>>>(f->work, b, a, f->plan[a], f->tw[a]);
+      launch_chained(k_f_lines<-1>, blocks, kFieldThreads, lines_smem(b.n[a]), f->stream, f->work, b, a, f->plan[a], f->tw[a]);
     else
-      k_f_lines<1><<<blocks, kFieldThreads, lines_smem(b.n[a]), f->stream>>>(f->work, b, a, f->plan[a], f->tw[a]);
+      launch_chained(k_f_lines<1>, blocks, kFieldThreads, lines_smem(b.n[a]), f->stream, f->work, b, a, f->plan[a], f->tw[a]);
   }
 }
 
@@ -518,10 +529,10 @@ int bg_fields_sphere_forward(bg_fields* f, const double* density, double* coeffs
     out = f->stage_c;
   }
   const unsigned g = (unsigned)std::min<int64_t>((total + 255) / 256, kFieldBlocks);
-  k_f_load_real<<<g, 256, 0, f->stream>>>(rho, total, f->work);
+  launch_chained(k_f_load_real, g, 256, 0, f->stream, rho, total, f->work);
   f_transform(f, -1);
   const unsigned gs = (unsigned)std::min<int64_t>((f->nsphere + 255) / 256, kFieldBlocks);
-  k_f_pick<<<gs, 256, 0, f->stream>>>(f->work, f->sphere, f->nsphere, 1.0 / (double)total, out);
+  launch_chained(k_f_pick, gs, 256, 0, f->stream, f->work, f->sphere, f->nsphere, 1.0 / (double)total, out);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
   if (ptr_kind == BG_PTR_HOST &&
       (e = cudaMemcpyAsync(coeffs, out, sizeof(double2) * f->nsphere, cudaMemcpyDeviceToHost, f->stream)) != cudaSuccess)
@@ -559,10 +570,10 @@ int bg_fields_sphere_inverse(bg_fields* f, const double* coeffs, double* density
   }
   const unsigned g = (unsigned)std::min<int64_t>((total + 255) / 256, kFieldBlocks);
   const unsigned gs = (unsigned)std::min<int64_t>((f->nsphere + 255) / 256, kFieldBlocks);
-  k_f_zero<<<g, 256, 0, f->stream>>>(f->work, total);
-  k_f_place<<<gs, 256, 0, f->stream>>>(c, f->sphere, f->nsphere, f->work, f->err);
+  launch_chained(k_f_zero, g, 256, 0, f->stream, f->work, total);
+  launch_chained(k_f_place, gs, 256, 0, f->stream, c, f->sphere, f->nsphere, f->work, f->err);
   f_transform(f, 1);
-  k_f_half_real<<<g, 256, 0, f->stream>>>(f->work, c, f->sphere_g0, total, rho);
+  launch_chained(k_f_half_real, g, 256, 0, f->stream, f->work, c, f->sphere_g0, total, rho);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
   if (ptr_kind == BG_PTR_HOST &&
       (e = cudaMemcpyAsync(density, rho, sizeof(double) * total, cudaMemcpyDeviceToHost, f->stream)) != cudaSuccess)

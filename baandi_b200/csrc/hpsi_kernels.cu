@@ -19,6 +19,7 @@
 // gather); crates/dft-physics/src/distributed_complex.rs:340-386 (complex apply);
 // crates/dft-physics/src/distributed_real_gamma.rs:654-689 (pair pack), :1307-1347
 // (unpack + kinetic), :957-1017, 1184-1248 (nonlocal).
+#include "launch_chain.cuh"
 #include "hpsi.h"
 #include "gemm_rns.cuh"
 #include "gemm_tc.cuh"
@@ -97,6 +98,7 @@ constexpr int sticks_blocks_per_sm() {
 
 template <bool GAMMA, int N, class C = double2>
 __global__ void __launch_bounds__(N == 0 ? 256 : 128, sticks_blocks_per_sm<N, C>()) k_sticks_inverse(const OpTables* __restrict__ tabs, BoxGeo g, Batch b) {
+  chain_wait();
   static_assert(N != 0 || sizeof(C) == sizeof(double2), "the runtime-plan engine is FP64 only");
   const OpTables& t = tabs[blockIdx.z];
   const CallArgs a = resolve(b.a[blockIdx.z]);
@@ -162,6 +164,7 @@ __global__ void __launch_bounds__(N == 0 ? 256 : 128, sticks_blocks_per_sm<N, C>
 // ---------------------------------------------------------------- pass 2
 // Planes with an axis outside fft_any.cuh (shorter than 15, or 125): runtime radices.
 __global__ void __launch_bounds__(512) k_planes(const OpTables* __restrict__ tabs, BoxGeo g, Batch b) {
+  chain_wait();
   const OpTables& t = tabs[blockIdx.z];
   const CallArgs a = resolve(b.a[blockIdx.z]);
   const int unit = blockIdx.x, z = blockIdx.y;
@@ -224,6 +227,7 @@ __host__ __device__ constexpr int planes_threads() {
 template <int N, class C = double2>
 __global__ void __launch_bounds__(planes_threads<N, C>(), planes_blocks_per_sm<N, C>())
     k_planes_fast(const OpTables* __restrict__ tabs, BoxGeo g, Batch b) {
+  chain_wait();
   using T = RealOf<C>;
   using Pl = fast::Plan<N>;
   static_assert(Pl::nst == 2, "two-stage plans");
@@ -295,6 +299,7 @@ __global__ void __launch_bounds__(planes_threads<N, C>(), planes_blocks_per_sm<N
 // ---------------------------------------------------------------- pass 3
 template <bool GAMMA, int N, class C = double2>
 __global__ void __launch_bounds__(N == 0 ? 256 : 128, sticks_blocks_per_sm<N, C>()) k_sticks_forward(const OpTables* __restrict__ tabs, BoxGeo g, Batch b) {
+  chain_wait();
   static_assert(N != 0 || sizeof(C) == sizeof(double2), "the runtime-plan engine is FP64 only");
   const OpTables& t = tabs[blockIdx.z];
   const CallArgs a = resolve(b.a[blockIdx.z]);
@@ -453,6 +458,7 @@ struct Ops<double2> {
 template <class T>
 __global__ void __launch_bounds__(256, 2) k_project(const NlDev* __restrict__ nls, int nproj, int ksplit,
                                                     int kchunk, Batch b) {
+  chain_wait();
   const int kb = blockIdx.z / ksplit, ks = blockIdx.z - kb * ksplit;
   const NlDev& nl = nls[kb];
   const CallArgs ca = resolve(b.a[kb]);
@@ -467,6 +473,7 @@ __global__ void __launch_bounds__(256, 2) k_project(const NlDev* __restrict__ nl
 // wd[c][off+i] = sum_j D[i][j] (sum_ks part[ks][c][off+j]) for one (atom, column).
 template <class T>
 __global__ void k_couple(const NlDev* __restrict__ nls, int nproj, int ksplit, Batch b) {
+  chain_wait();
   __shared__ T w[64];
   const NlDev& nl = nls[blockIdx.z];
   const int cols = resolve(b.a[blockIdx.z]).cols;
@@ -496,6 +503,7 @@ __global__ void k_couple(const NlDev* __restrict__ nls, int nproj, int ksplit, B
 // y[c][row] += sum_p P[p][row] wd[c][p]; tile 64 rows x 32 columns.
 template <class T>
 __global__ void __launch_bounds__(256, 2) k_back(const NlDev* __restrict__ nls, int nproj, Batch b) {
+  chain_wait();
   const NlDev& nl = nls[blockIdx.z];
   const CallArgs ca = resolve(b.a[blockIdx.z]);
   const int cols = ca.cols, rows = nl.rows;
@@ -525,6 +533,7 @@ template <int N>
 __global__ void __launch_bounds__(planes_threads<N, double2>(), planes_threads<N, double2>() == 512 ? 1 : 4)
     k_density_planes_fast(const OpTables* __restrict__ tabs, BoxGeo g, Batch b, int gamma, const double* __restrict__ w,
                           int wstride, int unit0, double* __restrict__ part) {
+  chain_wait();
   using Pl = fast::Plan<N>;
   static_assert(Pl::nst == 2, "two-stage plans");
   constexpr int R1 = Pl::radix[0], R2 = Pl::radix[1];
@@ -582,6 +591,7 @@ __global__ void __launch_bounds__(planes_threads<N, double2>(), planes_threads<N
 __global__ void __launch_bounds__(256, 1) k_density_planes(const OpTables* __restrict__ tabs, BoxGeo g, Batch b,
                                                         int gamma, const double* __restrict__ w, int wstride,
                                                         int unit0, double* __restrict__ part) {
+  chain_wait();
   const OpTables& t = tabs[blockIdx.z];
   const CallArgs& a = b.a[blockIdx.z];
   const int z = blockIdx.x, unit = unit0 + blockIdx.y;
@@ -619,6 +629,7 @@ __global__ void __launch_bounds__(256, 1) k_density_planes(const OpTables* __res
 // chains run side by side.
 __global__ void k_density_sum_chunks(const double* __restrict__ part, int chunks, int64_t total, double volume,
                                      int first, int last, double* __restrict__ ksum) {
+  chain_wait();
   const int k = blockIdx.y;
   const double* pk = part + (int64_t)k * chunks * total;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
@@ -633,6 +644,7 @@ __global__ void k_density_sum_chunks(const double* __restrict__ part, int chunks
 // (the arithmetic of one call per k point accumulating into out).
 __global__ void k_density_sum_k(const double* __restrict__ ksum, int nk, int n0, int n1, int n2, int accumulate,
                                 double* __restrict__ out) {
+  chain_wait();
   const int64_t pts = (int64_t)n0 * n1, total = pts * n2;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
     const int z = (int)(q / pts);
@@ -719,13 +731,13 @@ static void local_kernels(const OpTables* tabs, const BoxGeo& g, const Batch& b,
   if constexpr (N == 0 && sizeof(C) != sizeof(double2)) {
     return;  // the FP32 apply needs a compile-time plan (checked by the callers)
   } else {
-    { StageScope sc(ev, 0, s); k_sticks_inverse<GAMMA, N, C><<<sgrid, st, ss, s>>>(tabs, g, b); }
+    { StageScope sc(ev, 0, s); launch_chained(k_sticks_inverse<GAMMA, N, C>, sgrid, st, ss, s, tabs, g, b); }
     {
       StageScope sc(ev, 1, s);
       bool done = false;
       if constexpr (N != 0) {
         if (g.n0 == N && g.n1 == N) {
-          k_planes_fast<N, C><<<pgrid, planes_threads<N, C>(), ps, s>>>(tabs, g, b);
+          launch_chained(k_planes_fast<N, C>, pgrid, planes_threads<N, C>(), ps, s, tabs, g, b);
           done = true;
         }
       }
@@ -733,10 +745,10 @@ static void local_kernels(const OpTables* tabs, const BoxGeo& g, const Batch& b,
         if (!done && plane_any_supported(g))
           launch_planes_any(tabs, g, b, pgrid, s);
         else if (!done)
-          k_planes<<<pgrid, 512, ps, s>>>(tabs, g, b);
+          launch_chained(k_planes, pgrid, 512, ps, s, tabs, g, b);
       }
     }
-    { StageScope sc(ev, 2, s); k_sticks_forward<GAMMA, N, C><<<sgrid, st, ss, s>>>(tabs, g, b); }
+    { StageScope sc(ev, 2, s); launch_chained(k_sticks_forward<GAMMA, N, C>, sgrid, st, ss, s, tabs, g, b); }
   }
 }
 
@@ -807,9 +819,9 @@ static void density_sticks(const OpTables* tabs, int gamma, const BoxGeo& g, con
   constexpr int st = N == 0 ? 256 : 128;
   const size_t ss = stick_smem_bytes(g);
   if (gamma)
-    k_sticks_inverse<true, N><<<sgrid, st, ss, s>>>(tabs, g, b);
+    launch_chained(k_sticks_inverse<true, N>, sgrid, st, ss, s, tabs, g, b);
   else
-    k_sticks_inverse<false, N><<<sgrid, st, ss, s>>>(tabs, g, b);
+    launch_chained(k_sticks_inverse<false, N>, sgrid, st, ss, s, tabs, g, b);
 }
 
 template <int N>
@@ -818,7 +830,7 @@ static void density_planes(const OpTables* tabs, int gamma, const BoxGeo& g, con
   const size_t ds = density_smem_bytes(g);
   if constexpr (N != 0) {
     if (g.n0 == N && g.n1 == N) {
-      k_density_planes_fast<N><<<dgrid, planes_threads<N, double2>(), ds, s>>>(tabs, g, b, gamma, w, wstride, unit0,
+      launch_chained(k_density_planes_fast<N>, dgrid, planes_threads<N, double2>(), ds, s, tabs, g, b, gamma, w, wstride, unit0,
                                                                                part);
       return;
     }
@@ -826,7 +838,7 @@ static void density_planes(const OpTables* tabs, int gamma, const BoxGeo& g, con
   if (plane_any_supported(g))
     launch_density_any(tabs, g, b, gamma, w, wstride, unit0, part, dgrid, s);
   else
-    k_density_planes<<<dgrid, 256, ds, s>>>(tabs, g, b, gamma, w, wstride, unit0, part);
+    launch_chained(k_density_planes, dgrid, 256, ds, s, tabs, g, b, gamma, w, wstride, unit0, part);
 }
 
 int launch_density(const OpTables* tabs, int gamma, int max_groups, const BoxGeo& g, const Batch& b,
@@ -858,12 +870,12 @@ int launch_density(const OpTables* tabs, int gamma, int max_groups, const BoxGeo
 #define BG_PLANES(NN) density_planes<NN>(tabs, gamma, g, b, weights, wstride, u0, part, dgrid, s)
     BG_DENS(BG_PLANES)
 #undef BG_PLANES
-    k_density_sum_chunks<<<dim3(bx, b.nk), 256, 0, s>>>(part, n, total, volume, u0 == 0, u0 + n >= max_units, ksum);
+    launch_chained(k_density_sum_chunks, dim3(bx, b.nk), 256, 0, s, part, n, total, volume, u0 == 0, u0 + n >= max_units, ksum);
     launches += 2;
   }
 #undef BG_DENS
   const int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 8);
-  k_density_sum_k<<<blocks, 256, 0, s>>>(ksum, b.nk, g.n0, g.n1, g.n2, accumulate, out);
+  launch_chained(k_density_sum_k, blocks, 256, 0, s, ksum, b.nk, g.n0, g.n1, g.n2, accumulate, out);
   return launches;
 }
 
@@ -909,19 +921,19 @@ int launch_nonlocal(const NlDev* nl, int gamma, const NlShape& sh, int max_rows,
   if (gamma) {
     {
       StageScope sc(ev, 3, s);
-      k_project<double><<<pg, 256, tiles::tn48m_smem_bytes<double>(), s>>>(nl, sh.nproj, sh.ksplit, sh.kchunk, b);
+      launch_chained(k_project<double>, pg, 256, tiles::tn48m_smem_bytes<double>(), s, nl, sh.nproj, sh.ksplit, sh.kchunk, b);
     }
-    { StageScope sc(ev, 4, s); k_couple<double><<<cg, cth, 0, s>>>(nl, sh.nproj, sh.ksplit, b); }
-    { StageScope sc(ev, 5, s); k_back<double><<<bg_, 256, tiles::nn64m_smem_bytes<double>(), s>>>(nl, sh.nproj, b); }
+    { StageScope sc(ev, 4, s); launch_chained(k_couple<double>, cg, cth, 0, s, nl, sh.nproj, sh.ksplit, b); }
+    { StageScope sc(ev, 5, s); launch_chained(k_back<double>, bg_, 256, tiles::nn64m_smem_bytes<double>(), s, nl, sh.nproj, b); }
   } else {
     {
       StageScope sc(ev, 3, s);
-      k_project<double2><<<pg, 256, tiles::tn48m_smem_bytes<double2>(), s>>>(nl, sh.nproj, sh.ksplit, sh.kchunk, b);
+      launch_chained(k_project<double2>, pg, 256, tiles::tn48m_smem_bytes<double2>(), s, nl, sh.nproj, sh.ksplit, sh.kchunk, b);
     }
-    { StageScope sc(ev, 4, s); k_couple<double2><<<cg, cth, 0, s>>>(nl, sh.nproj, sh.ksplit, b); }
+    { StageScope sc(ev, 4, s); launch_chained(k_couple<double2>, cg, cth, 0, s, nl, sh.nproj, sh.ksplit, b); }
     {
       StageScope sc(ev, 5, s);
-      k_back<double2><<<bg_, 256, tiles::nn64m_smem_bytes<double2>(), s>>>(nl, sh.nproj, b);
+      launch_chained(k_back<double2>, bg_, 256, tiles::nn64m_smem_bytes<double2>(), s, nl, sh.nproj, b);
     }
   }
   return 3;
@@ -998,6 +1010,7 @@ int configure_kernels(size_t plane_smem, size_t stick_smem) {
 // [k] P^H x into the projection buffer, [nk + k] y += P wd, P from the operator's
 // split panels.  One thread per operator.
 __global__ void k_nl_tc_descs(const NlDev* __restrict__ nls, int nproj, Batch b, tc::ZDesc* __restrict__ out) {
+  chain_wait();
   const int k = threadIdx.x;
   if (k >= b.nk) return;
   const NlDev& nl = nls[k];
@@ -1046,6 +1059,7 @@ int ensure_nonlocal_tc(TcNl* t, int nk, int nproj, int max_cols, int max_rows) {
 // Descriptors of the FP64 residue products of every operator of a batch: [k] P^H x into the
 // projection buffer, [nk + k] y += P wd.  One thread per operator.
 __global__ void k_nl_rns_descs(const NlDev* __restrict__ nls, int nproj, Batch b, rns::Desc* __restrict__ out) {
+  chain_wait();
   const int k = threadIdx.x;
   if (k >= b.nk) return;
   const NlDev& nl = nls[k];
@@ -1094,7 +1108,7 @@ int launch_nonlocal_rns(const NlDev* nl, const NlShape& sh, int max_rows, int ma
   if (sh.nproj == 0 || max_cols == 0 || b.nk == 0) return 0;
   rns::Desc* d = static_cast<rns::Desc*>(r->desc);
   int launches = 2;
-  k_nl_rns_descs<<<1, kMaxBatch, 0, s>>>(nl, sh.nproj, b, d);
+  launch_chained(k_nl_rns_descs, 1, kMaxBatch, 0, s, nl, sh.nproj, b, d);
   {
     StageScope sc(ev, 3, s);
     launches += rns::launch_product(rns::kTN, d, b.nk, sh.nproj, max_cols, max_rows, true, r->work, r->bytes, err, s);
@@ -1102,7 +1116,7 @@ int launch_nonlocal_rns(const NlDev* nl, const NlShape& sh, int max_rows, int ma
   {
     StageScope sc(ev, 4, s);
     const dim3 cg(sh.natoms, max_cols, b.nk);
-    k_couple<double2><<<cg, ((sh.maxch + 31) / 32) * 32, 0, s>>>(nl, sh.nproj, 1, b);
+    launch_chained(k_couple<double2>, cg, ((sh.maxch + 31) / 32) * 32, 0, s, nl, sh.nproj, 1, b);
   }
   {
     StageScope sc(ev, 5, s);
@@ -1116,7 +1130,7 @@ int launch_nonlocal_tc(const NlDev* nl, const NlShape& sh, int max_rows, int max
   if (sh.nproj == 0 || max_cols == 0 || b.nk == 0) return 0;
   tc::ZDesc* d = static_cast<tc::ZDesc*>(t->desc);
   int launches = 1;
-  k_nl_tc_descs<<<1, kMaxBatch, 0, s>>>(nl, sh.nproj, b, d);
+  launch_chained(k_nl_tc_descs, 1, kMaxBatch, 0, s, nl, sh.nproj, b, d);
   {
     StageScope sc(ev, 3, s);
     launches += tc::launch_zgemm(tc::kTN, d, b.nk, sh.nproj, max_cols, max_rows, t->ksplit, true, t->work, t->err, s);
@@ -1124,7 +1138,7 @@ int launch_nonlocal_tc(const NlDev* nl, const NlShape& sh, int max_rows, int max
   {
     StageScope sc(ev, 4, s);
     const dim3 cg(sh.natoms, max_cols, b.nk);
-    k_couple<double2><<<cg, ((sh.maxch + 31) / 32) * 32, 0, s>>>(nl, sh.nproj, 1, b);
+    launch_chained(k_couple<double2>, cg, ((sh.maxch + 31) / 32) * 32, 0, s, nl, sh.nproj, 1, b);
     launches += 1;
   }
   {

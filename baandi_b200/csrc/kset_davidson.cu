@@ -27,6 +27,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "launch_chain.cuh"
 #include "blas_dev.cuh"
 #include "gemm_rns.cuh"
 #include "gemm_tc.cuh"
@@ -581,6 +582,7 @@ __device__ bool eigen(const Bufs<D>& b, int cap, int m, double* red, int* sh) {
 template <class D>
 __global__ void __launch_bounds__(256, 2) k_dv_nn(const Bufs<D>* __restrict__ bufs, const NN<D>* __restrict__ desc,
                                                   int nk, int residues) {
+  chain_wait();
   const int z = blockIdx.z, k = z % nk;
   const NN<D> d = desc[z];
   const int rows = bufs[k].rows;
@@ -596,6 +598,7 @@ __global__ void __launch_bounds__(256, 2) k_dv_nn(const Bufs<D>* __restrict__ bu
 template <class D>
 __global__ void __launch_bounds__(256, 2) k_dv_tn(const Bufs<D>* __restrict__ bufs, const TN<D>* __restrict__ desc, int nk,
                                               int ks, int64_t slot_elems, int residues) {
+  chain_wait();
   const int zz = blockIdx.z / ks, sidx = blockIdx.z % ks;
   const int slot = zz / nk, k = zz % nk;
   const TN<D> d = desc[zz];
@@ -613,6 +616,7 @@ __global__ void __launch_bounds__(256, 2) k_dv_tn(const Bufs<D>* __restrict__ bu
 template <class D>
 __global__ void k_dv_tn_sum(const Bufs<D>* __restrict__ bufs, const TN<D>* __restrict__ desc, int nk, int ks,
                             int64_t slot_elems, int residues) {
+  chain_wait();
   const int zz = blockIdx.z, slot = zz / nk, k = zz % nk;
   const TN<D> d = desc[zz];
   if (d.m <= 0 || d.n <= 0 || d.prec || (residues && rns::pays(d.m, d.n, bufs[k].rows, false))) return;
@@ -632,6 +636,7 @@ __global__ void k_dv_tn_sum(const Bufs<D>* __restrict__ bufs, const TN<D>* __res
 constexpr int kCopyUnroll = 4;
 template <class D>
 __global__ void k_dv_copy(const Bufs<D>* __restrict__ bufs, const CP<D>* __restrict__ desc, int nk) {
+  chain_wait();
   const int z = blockIdx.z, k = z % nk;
   const CP<D> d = desc[z];
   const int c = blockIdx.y;
@@ -677,6 +682,7 @@ template <class D>
 __global__ void __launch_bounds__(256) k_dv_corrections(const Bufs<D>* __restrict__ bufs, const Ctl* __restrict__ ctl,
                                                         const Opts* __restrict__ opts,
                                                         const __nv_bfloat16* __restrict__ net) {
+  chain_wait();
   __shared__ double red[256];
   __shared__ float wnet[learned::kParams];
   const int j = blockIdx.x, k = blockIdx.y;
@@ -706,6 +712,7 @@ __global__ void __launch_bounds__(256) k_dv_corrections(const Bufs<D>* __restric
 template <class D>
 __global__ void k_dv_tc_descs(const Bufs<D>* __restrict__ bufs, const NN<D>* __restrict__ nn, int n_nn,
                               const TN<D>* __restrict__ tn, int n_tn, int nk, tc::ZDesc* out_nn, tc::ZDesc* out_tn) {
+  chain_wait();
   const int z = blockIdx.x * blockDim.x + threadIdx.x;
   const tc::ZDesc empty{nullptr, nullptr, nullptr, 1, 1, 1, 0, 0, 0, tc::kStore};
   if (z < n_nn * nk) {
@@ -732,6 +739,7 @@ __global__ void k_dv_tc_descs(const Bufs<D>* __restrict__ bufs, const NN<D>* __r
 template <class D>
 __global__ void k_dv_rns_descs(const Bufs<D>* __restrict__ bufs, const NN<D>* __restrict__ nn, int n_nn,
                                const TN<D>* __restrict__ tn, int n_tn, int nk, rns::Desc* out) {
+  chain_wait();
   const int z = blockIdx.x * blockDim.x + threadIdx.x;
   rns::Desc o{nullptr, nullptr, nullptr, 1, 1, 1, 0, 0, 0, rns::kStore};
   if (z < n_nn * nk) {
@@ -790,6 +798,7 @@ template <class D>
 __global__ void __launch_bounds__(kCtlThreads, 1) k_dv_ctl(int phase, Bufs<D>* __restrict__ bufs, Ctl* ctl,
                                                         NN<D>* nn, TN<D>* tn, CP<D>* cp, DynCols* dyn,
                                                         const Opts* __restrict__ opts, int nk, int gamma) {
+  chain_wait();
   using X = Cx<D>;
   const Opts o = *opts;
   const int k = blockIdx.x;
@@ -1330,6 +1339,7 @@ struct IoPtrs {
 // pointers: one launch instead of six stream operations per k point.  blockIdx.y = k.
 template <class D>
 __global__ void k_dv_init(const Bufs<D>* __restrict__ bufs, const IoPtrs* __restrict__ io, int n, int cap) {
+  chain_wait();
   const int k = blockIdx.y;
   const Bufs<D>& b = bufs[k];
   const int64_t cc = (int64_t)cap * cap, rn = (int64_t)b.rows * n;
@@ -1358,6 +1368,7 @@ __global__ void k_dv_init(const Bufs<D>* __restrict__ bufs, const IoPtrs* __rest
 template <class D>
 __global__ void k_dv_out(const Bufs<D>* __restrict__ bufs, const IoPtrs* __restrict__ io, int n, int nk,
                          double* __restrict__ out) {
+  chain_wait();
   const int k = blockIdx.y;
   const Bufs<D>& b = bufs[k];
   const IoPtrs p = io[k];
@@ -1521,7 +1532,7 @@ class KsetSolver {
   static bool small(int cap) { return vec_smem(cap) + mat_smem(cap) <= 200 * 1024; }
   size_t ctl_smem() const { return vec_smem(o_.cap) + (o_.smem_matrices ? mat_smem(o_.cap) : 0); }
   int64_t ctl(int phase) {
-    k_dv_ctl<D><<<nk_, kCtlThreads, ctl_smem(), s_>>>(phase, d_bufs_, d_ctl_, d_nn_, d_tn_, d_cp_, d_dyn_, d_opts_,
+    launch_chained(k_dv_ctl<D>, nk_, kCtlThreads, ctl_smem(), s_, phase, d_bufs_, d_ctl_, d_nn_, d_tn_, d_cp_, d_dyn_, d_opts_,
                                                      nk_, ks_->gamma);
     return 1;
   }
@@ -1530,15 +1541,15 @@ class KsetSolver {
   int64_t nn(int nslots, bool residues = true) {
     const dim3 grid((unsigned)((o_.cap + 63) / 64), (unsigned)((max_rows_ + 63) / 64), (unsigned)(nslots * nk_));
     residues = residues && rns_work_;
-    k_dv_nn<D><<<grid, 256, tiles::nn64m_smem_bytes<D>(), s_>>>(d_bufs_, d_nn_, nk_, residues ? 1 : 0);
+    launch_chained(k_dv_nn<D>, grid, 256, tiles::nn64m_smem_bytes<D>(), s_, d_bufs_, d_nn_, nk_, residues ? 1 : 0);
     int64_t l = 1;
     if (residues) {
-      k_dv_rns_descs<D><<<1, 128, 0, s_>>>(d_bufs_, d_nn_, nslots, d_tn_, 0, nk_, d_rns_);
+      launch_chained(k_dv_rns_descs<D>, 1, 128, 0, s_, d_bufs_, d_nn_, nslots, d_tn_, 0, nk_, d_rns_);
       l += 1 + rns::launch_product(rns::kNN, d_rns_, nslots * nk_, max_rows_, o_.n, o_.cap, false, rns_work_, rns_bytes_,
                                    ks_->ops[0]->t.err, s_);
     }
     if (!tensor_products()) return l;
-    k_dv_tc_descs<D><<<1, 128, 0, s_>>>(d_bufs_, d_nn_, nslots, d_tn_, 0, nk_, d_tcnn_, d_tctn_);
+    launch_chained(k_dv_tc_descs<D>, 1, 128, 0, s_, d_bufs_, d_nn_, nslots, d_tn_, 0, nk_, d_tcnn_, d_tctn_);
     return l + 1 + tc::launch_zgemm(tc::kNN, d_tcnn_, nslots * nk_, max_rows_, o_.cap, o_.cap, 1, false, tc_work_,
                                 tc_err_, s_);
   }
@@ -1546,19 +1557,19 @@ class KsetSolver {
   int64_t tn(int nslots, bool residues = true) {
     const unsigned t = (unsigned)((o_.cap + 47) / 48);
     residues = residues && rns_work_;
-    k_dv_tn<D><<<dim3(t, t, (unsigned)(nslots * nk_ * ksplit_)), 256, tiles::tn48m_smem_bytes<D>(), s_>>>(
+    launch_chained(k_dv_tn<D>, dim3(t, t, (unsigned)(nslots * nk_ * ksplit_)), 256, tiles::tn48m_smem_bytes<D>(), s_, 
         d_bufs_, d_tn_, nk_, ksplit_, slot_elems_, residues ? 1 : 0);
     const unsigned blocks = (unsigned)std::min<int64_t>(((int64_t)o_.cap * o_.cap + 255) / 256, 64);
-    k_dv_tn_sum<D><<<dim3(blocks, 1, (unsigned)(nslots * nk_)), 256, 0, s_>>>(d_bufs_, d_tn_, nk_, ksplit_,
+    launch_chained(k_dv_tn_sum<D>, dim3(blocks, 1, (unsigned)(nslots * nk_)), 256, 0, s_, d_bufs_, d_tn_, nk_, ksplit_,
                                                                               slot_elems_, residues ? 1 : 0);
     int64_t l = 2;
     if (residues) {
-      k_dv_rns_descs<D><<<1, 128, 0, s_>>>(d_bufs_, d_nn_, 0, d_tn_, nslots, nk_, d_rns_);
+      launch_chained(k_dv_rns_descs<D>, 1, 128, 0, s_, d_bufs_, d_nn_, 0, d_tn_, nslots, nk_, d_rns_);
       l += 1 + rns::launch_product(rns::kTN, d_rns_, nslots * nk_, o_.cap, o_.n, max_rows_, false, rns_work_, rns_bytes_,
                                    ks_->ops[0]->t.err, s_);
     }
     if (!tensor_products()) return l;
-    k_dv_tc_descs<D><<<1, 128, 0, s_>>>(d_bufs_, d_nn_, 0, d_tn_, nslots, nk_, d_tcnn_, d_tctn_);
+    launch_chained(k_dv_tc_descs<D>, 1, 128, 0, s_, d_bufs_, d_nn_, 0, d_tn_, nslots, nk_, d_tcnn_, d_tctn_);
     return l + 1 + tc::launch_zgemm(tc::kTN, d_tctn_, nslots * nk_, o_.cap, o_.cap, max_rows_, tc_ks_, false, tc_work_,
                                 tc_err_, s_);
   }
@@ -1618,11 +1629,11 @@ class KsetSolver {
     const int64_t span = 256 * kCopyUnroll;
     const dim3 grid((unsigned)std::min<int64_t>((max_rows_ + span - 1) / span, 64), (unsigned)o_.cap,
                     (unsigned)(nslots * nk_));
-    k_dv_copy<D><<<grid, 256, 0, s_>>>(d_bufs_, d_cp_ + (size_t)slot0 * nk_, nk_);
+    launch_chained(k_dv_copy<D>, grid, 256, 0, s_, d_bufs_, d_cp_ + (size_t)slot0 * nk_, nk_);
     return 1;
   }
   int64_t corr() {
-    k_dv_corrections<D><<<dim3((unsigned)o_.n, (unsigned)nk_), 256, 0, s_>>>(
+    launch_chained(k_dv_corrections<D>, dim3((unsigned)o_.n, (unsigned)nk_), 256, 0, s_, 
         d_bufs_, d_ctl_, d_opts_, static_cast<const __nv_bfloat16*>(ks_->ctx->learned));
     return 1;
   }
@@ -1798,7 +1809,7 @@ int KsetSolver<T>::run(const double* const* start, const double* const* diagonal
   }
   if ((rc = cuda(cudaMemcpyAsync(d_io_, h_io_, sizeof(IoPtrs) * nk_, cudaMemcpyHostToDevice, s_), "upload")))
     return rc;
-  k_dv_init<D><<<dim3(64, nk_), 256, 0, s_>>>(d_bufs_, d_io_, n, cap);
+  launch_chained(k_dv_init<D>, dim3(64, nk_), 256, 0, s_, d_bufs_, d_io_, n, cap);
   launches_ += 1;
   if ((rc = cuda(cudaMemcpyAsync(d_opts_, &o_, sizeof(Opts), cudaMemcpyHostToDevice, s_), "upload"))) return rc;
   // start: H V and the Grams of the start block, descriptors written from the host
@@ -1865,7 +1876,7 @@ int KsetSolver<T>::run(const double* const* start, const double* const* diagonal
   // contractions exchange V and X (and HV and HX) on the device: refresh the host mirror
   if ((rc = cuda(cudaMemcpy(hb_.data(), d_bufs_, sizeof(Bufs<D>) * nk_, cudaMemcpyDeviceToHost), "buffers")))
     return rc;
-  k_dv_out<D><<<dim3(64, nk_), 256, 0, s_>>>(d_bufs_, d_io_, n, nk_, d_out_);
+  launch_chained(k_dv_out<D>, dim3(64, nk_), 256, 0, s_, d_bufs_, d_io_, n, nk_, d_out_);
   launches_ += 1;
   const size_t outn = (size_t)nk_ * (2 * n + 1);
   if ((rc = cuda(cudaMemcpyAsync(h_out_, d_out_, sizeof(double) * outn, cudaMemcpyDeviceToHost, s_), "copy out")))

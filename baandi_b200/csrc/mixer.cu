@@ -21,6 +21,7 @@
 #include <string>
 #include <vector>
 
+#include "launch_chain.cuh"
 #include "op_internal.h"
 
 namespace bg {
@@ -43,6 +44,7 @@ __device__ __forceinline__ void neu_add(Neu& a, double v) {
 
 __global__ void k_mix_diff(const double2* __restrict__ x, const double2* __restrict__ f, double2* prev_x,
                            double2* prev_f, double2* __restrict__ dx, double2* __restrict__ df, int64_t n, int have_slot) {
+  chain_wait();
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
     const double2 xv = x[j], fv = f[j];
     if (have_slot) {
@@ -60,6 +62,7 @@ __global__ void k_mix_diff(const double2* __restrict__ x, const double2* __restr
 __global__ void __launch_bounds__(kMixThreads) k_mix_forms(const double2* __restrict__ df, int64_t n, int p,
                                                            const double2* __restrict__ f,
                                                            const double* __restrict__ w, double* __restrict__ forms) {
+  chain_wait();
   const int q = blockIdx.x;
   const int tri = p * (p + 1) / 2;
   const double2* a;
@@ -100,6 +103,7 @@ __global__ void __launch_bounds__(kMixThreads) k_mix_forms(const double2* __rest
 // out[2] = lambda_max, out[3] = condition.
 __global__ void k_mix_solve(const double* __restrict__ forms, int p, double* __restrict__ gamma,
                             double* __restrict__ out) {
+  chain_wait();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   double A[kMaxHistory][kMaxHistory], Q[kMaxHistory][kMaxHistory];
   int idx = 0;
@@ -180,6 +184,7 @@ __global__ void k_mix_apply(const double2* __restrict__ x, const double2* __rest
                             const double* __restrict__ gamma, const int* __restrict__ smooth,
                             const double* __restrict__ screening, double beta, double2* __restrict__ next,
                             double2* __restrict__ reduced, int* err) {
+  chain_wait();
   __shared__ double g[kMaxHistory];
   if ((int)threadIdx.x < p) g[threadIdx.x] = gamma[threadIdx.x];
   __syncthreads();
@@ -354,11 +359,11 @@ int bg_mixer_update(bg_mixer* m, const double* x, const double* f, double* next,
   const int slot = it > 1 ? (it - 2) % m->history : -1;
   const int p = std::min(std::max(it - 1, 0), m->history);
   const unsigned gb = grid_for(n);
-  k_mix_diff<<<gb, 256, 0, m->stream>>>(dxp, dfp, m->prev_x, m->prev_f, m->dx + (slot < 0 ? 0 : (int64_t)slot * n),
+  launch_chained(k_mix_diff, gb, 256, 0, m->stream, dxp, dfp, m->prev_x, m->prev_f, m->dx + (slot < 0 ? 0 : (int64_t)slot * n),
                                         m->df + (slot < 0 ? 0 : (int64_t)slot * n), n, slot >= 0 ? 1 : 0);
   if (p > 0) {
-    k_mix_forms<<<p * (p + 1) / 2 + p, kMixThreads, 0, m->stream>>>(m->df, n, p, dfp, m->w, m->forms);
-    k_mix_solve<<<1, 32, 0, m->stream>>>(m->forms, p, m->gamma, m->out);
+    launch_chained(k_mix_forms, p * (p + 1) / 2 + p, kMixThreads, 0, m->stream, m->df, n, p, dfp, m->w, m->forms);
+    launch_chained(k_mix_solve, 1, 32, 0, m->stream, m->forms, p, m->gamma, m->out);
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
   double* h = m->host_out;
@@ -378,7 +383,7 @@ int bg_mixer_update(bg_mixer* m, const double* x, const double* f, double* next,
       return fail(ctx, BG_EINVAL, msg);
     }
   }
-  k_mix_apply<<<gb, 256, 0, m->stream>>>(dxp, dfp, m->dx, m->df, n, p, m->gamma, m->smooth, m->screening, m->beta,
+  launch_chained(k_mix_apply, gb, 256, 0, m->stream, dxp, dfp, m->dx, m->df, n, p, m->gamma, m->smooth, m->screening, m->beta,
                                          dnext, m->reduced, m->err);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
   if (ptr_kind == BG_PTR_HOST && (e = cudaMemcpyAsync(next, dnext, bytes, cudaMemcpyDeviceToHost, m->stream)) != cudaSuccess)
@@ -448,7 +453,7 @@ int bg_mixer_metric(bg_mixer* m, const double* a, const double* b, double* out, 
   }
   // one form: <a, b> = the right-hand side slot of a p = 1 batch with dF_0 := a
   double* tmp = m->out + 4;
-  k_mix_forms<<<1, kMixThreads, 0, m->stream>>>(da, n, 0, db, m->w, tmp);
+  launch_chained(k_mix_forms, 1, kMixThreads, 0, m->stream, da, n, 0, db, m->w, tmp);
   if ((e = cudaMemcpyAsync(m->host_out + 36, tmp, sizeof(double), cudaMemcpyDeviceToHost, m->stream)) != cudaSuccess ||
       (e = cudaStreamSynchronize(m->stream)) != cudaSuccess)
     return cuda_fail(ctx, e, "metric");

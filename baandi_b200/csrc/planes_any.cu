@@ -7,6 +7,7 @@
 // 147 us where the radix-2-to-5 runtime kernel (block barriers between four to six stages, the
 // plane cleared and scattered first) took 596 us; an engine with the length read inside its
 // stages took 470 us.
+#include "launch_chain.cuh"
 #include "plane_passes.cuh"
 
 #include "fft_any.cuh"
@@ -42,6 +43,7 @@ template <bool VS, int W>
 __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1) k_planes_any(const OpTables* __restrict__ tabs,
                                                                const __grid_constant__ BoxGeo g,
                                                                const __grid_constant__ Batch b) {
+  chain_wait();
   const OpTables& t = tabs[blockIdx.z];
   const CallArgs a = resolve(b.a[blockIdx.z]);
   const int unit = blockIdx.x, z = blockIdx.y;
@@ -84,6 +86,7 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1)
     k_density_planes_any(const OpTables* __restrict__ tabs, const __grid_constant__ BoxGeo g,
                          const __grid_constant__ Batch b, int gamma, const double* __restrict__ w, int wstride,
                          int unit0, double* __restrict__ part) {
+  chain_wait();
   const OpTables& t = tabs[blockIdx.z];
   const CallArgs& a = b.a[blockIdx.z];
   const int z = blockIdx.x, unit = unit0 + blockIdx.y;
@@ -136,22 +139,22 @@ void launch_planes_any(const OpTables* tabs, const BoxGeo& g, const Batch& b, di
   // the potential beside the plane where it costs no block
   if (any_warps(g) == 8) {
     if (any_smem(g, true) <= kPlaneAnyPair)
-      k_planes_any<true, 8><<<grid, 256, any_smem(g, true), s>>>(tabs, g, b);
+      launch_chained(k_planes_any<true, 8>, grid, 256, any_smem(g, true), s, tabs, g, b);
     else
-      k_planes_any<false, 8><<<grid, 256, any_smem(g, false), s>>>(tabs, g, b);
+      launch_chained(k_planes_any<false, 8>, grid, 256, any_smem(g, false), s, tabs, g, b);
   } else if (any_smem(g, true) <= kPlaneAnyMost) {
-    k_planes_any<true, 16><<<grid, 512, any_smem(g, true), s>>>(tabs, g, b);
+    launch_chained(k_planes_any<true, 16>, grid, 512, any_smem(g, true), s, tabs, g, b);
   } else {
-    k_planes_any<false, 16><<<grid, 512, any_smem(g, false), s>>>(tabs, g, b);
+    launch_chained(k_planes_any<false, 16>, grid, 512, any_smem(g, false), s, tabs, g, b);
   }
 }
 
 void launch_density_any(const OpTables* tabs, const BoxGeo& g, const Batch& b, int gamma, const double* w, int wstride,
                         int unit0, double* part, dim3 grid, cudaStream_t s) {
   if (any_warps(g) == 8)
-    k_density_planes_any<8><<<grid, 256, any_smem(g, false), s>>>(tabs, g, b, gamma, w, wstride, unit0, part);
+    launch_chained(k_density_planes_any<8>, grid, 256, any_smem(g, false), s, tabs, g, b, gamma, w, wstride, unit0, part);
   else
-    k_density_planes_any<16><<<grid, 512, any_smem(g, false), s>>>(tabs, g, b, gamma, w, wstride, unit0, part);
+    launch_chained(k_density_planes_any<16>, grid, 512, any_smem(g, false), s, tabs, g, b, gamma, w, wstride, unit0, part);
 }
 
 int configure_planes_any() {
