@@ -523,14 +523,23 @@ __global__ void __launch_bounds__(256, 2) k_back(const NlDev* __restrict__ nls, 
 // Reference: crates/dft-physics/src/distributed_complex.rs:485-547 (complex, sum in
 // band order of weight |u(r)|^2 / volume), distributed_real_gamma.rs:744-785 (Gamma
 // pairs: weight_a Re^2 + weight_b Im^2).
+// Density blocks per SM from their shared memory (no potential), at most 4.
+template <int N>
+constexpr int density_blocks_per_sm() {
+  const int bytes = (int)sizeof(double2) * (N + N * (N | 1)) + 4 * N;
+  const int fit = 233472 / (bytes + 16 * N + 1024);
+  return fit < 1 ? 1 : (fit > 4 ? 4 : fit);
+}
+
 // Tuned cubic lengths, one unit per (z plane, unit of the group, k point) block: the y inverse
 // on the x rows holding sticks (first stage straight from the stick row), the x inverse on
 // every column y (rows without sticks are zero and not loaded), then w |psi|^2 to the block's
-// own slice.  Blocks as k_planes_fast's: 64 registers up to 72^3, sixteen warps at 108^3.  (A
+// own slice.  Registers as the planes' shared memory allows: four blocks per SM up to 54^3, three
+// at 60^3, two at 72^3, one of sixteen warps at 108^3.  (A
 // block looping over units and adding into its slice held every stage's indices, 255 registers
 // and one block of eight warps: 11.0 ms for the 480 Si216 bands.)
 template <int N>
-__global__ void __launch_bounds__(planes_threads<N, double2>(), planes_threads<N, double2>() == 512 ? 1 : 4)
+__global__ void __launch_bounds__(planes_threads<N, double2>(), density_blocks_per_sm<N>())
     k_density_planes_fast(const OpTables* __restrict__ tabs, BoxGeo g, Batch b, int gamma, const double* __restrict__ w,
                           int wstride, int unit0, double* __restrict__ part) {
   chain_wait();
