@@ -981,8 +981,13 @@ static void configure_one(cudaError_t& e, size_t plane_smem, size_t stick_smem) 
   }
 }
 
+// The attributes live in the device's context: about 150 calls (1 ms) that an operator after
+// the first finds made, by the attribute of the kernel set last.
 int configure_kernels(size_t plane_smem, size_t stick_smem) {
-  cudaError_t e = cudaSuccess;
+  cudaFuncAttributes last{};
+  cudaError_t e = cudaFuncGetAttributes(&last, (const void*)k_sticks_forward<false, 108, float2>);
+  if (e != cudaSuccess) return 1;
+  if (last.maxDynamicSharedSizeBytes == (int)stick_smem && last.preferredShmemCarveout == 100) return 0;
   e = cudaFuncSetAttribute((const void*)k_project<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)tiles::tn48m_smem_bytes<double>());
   if (e == cudaSuccess)
