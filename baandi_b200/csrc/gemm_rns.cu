@@ -749,8 +749,10 @@ __global__ void __launch_bounds__(128) k_rns_join(const Desc* __restrict__ descs
       const int j = 4 * jc + c;
       if (j >= d.N) break;
       const double fr = (reh[c] - rint(reh[c])) + rel[c], fi = (imh[c] - rint(imh[c])) + iml[c];
-      const double vr = fma(fr, c_tab.mlo, fr * c_tab.mhi) * ai * binv[j];
-      const double vi = fma(fi, c_tab.mlo, fi * c_tab.mhi) * ai * binv[j];
+      // the smaller scale first: no overflow before the larger one (a NaN reaches the product)
+      const double bj = binv[j], s1 = ai < bj ? ai : bj, s2 = ai < bj ? bj : ai;
+      const double vr = fma(fr, c_tab.mlo, fr * c_tab.mhi) * s1 * s2;
+      const double vi = fma(fi, c_tab.mlo, fi * c_tab.mhi) * s1 * s2;
       double2* out = d.C + row + (int64_t)j * d.ldc;
       if (d.op == kStore) {
         *out = make_double2(vr, vi);
