@@ -69,7 +69,8 @@ def test_tile_edges(mode, m, n, k):
 
 
 @pytest.mark.parametrize("mode", [0, 1])
-def test_scales_and_nonfinite(mode):
+@pytest.mark.parametrize("power", [660, 940])   # 940: one scale alone overflows the intermediate
+def test_scales_and_nonfinite(mode, power):
     torch = pytest.importorskip("torch")
     m, n, k = 130, 33, 200
     a, b, c0 = matrices(mode, m, n, k, 5)
@@ -78,7 +79,7 @@ def test_scales_and_nonfinite(mode):
     b[1] = 0.0
     want, norms = exact(mode, a, b)
     ea, eb = np.zeros(m, np.int64), np.zeros(n, np.int64)
-    ea[0], ea[1], eb[0] = 660, -660, -660   # squares overflow and underflow; one product vanishes
+    ea[0], ea[1], eb[0] = power, -power, -power   # squares overflow and underflow; one product vanishes
     rows *= np.ldexp(1.0, ea)[:, None]
     b *= np.ldexp(1.0, eb)[:, None]
     rows[5, 11] = np.inf
