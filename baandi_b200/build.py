@@ -9,6 +9,8 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -46,13 +48,22 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not stale():
         return LIB
     tmp = LIB + ".tmp"
-    cmd = [nvcc(), *NVCC_FLAGS, "-shared", "-o", tmp] + [os.path.join(CSRC, s) for s in SOURCES] + ["-lcudart", "-lgomp"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
+    with tempfile.TemporaryDirectory() as work, ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+        objects = [os.path.join(work, s + ".o") for s in SOURCES]
+
+        def compile_one(args):
+            src, obj = args
+            return subprocess.run([nvcc(), *NVCC_FLAGS, "-c", "-o", obj, os.path.join(CSRC, src)], capture_output=True,
+                                  text=True)
+        done = list(pool.map(compile_one, zip(SOURCES, objects)))
+        if all(r.returncode == 0 for r in done):
+            done.append(subprocess.run([nvcc(), *NVCC_FLAGS, "-shared", "-o", tmp, *objects, "-lcudart", "-lgomp"],
+                                       capture_output=True, text=True))
+    if any(r.returncode != 0 for r in done):
+        sys.stderr.write("".join(r.stdout + r.stderr for r in done if r.returncode != 0))
         raise RuntimeError("nvcc failed building libbaandi_b200.so")
     if verbose:
-        sys.stderr.write(res.stderr)
+        sys.stderr.write("".join(r.stderr for r in done))
     os.replace(tmp, LIB)
     return LIB
 
