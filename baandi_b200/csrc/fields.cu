@@ -76,9 +76,9 @@ __device__ __forceinline__ double block_sum(double v, double* sm) {
   return r;
 }
 
-__global__ void __launch_bounds__(kFieldThreads) k_f_xc(const double* __restrict__ rho, int64_t total,
-                                                        double* __restrict__ vxc, double2* __restrict__ work,
-                                                        double* __restrict__ part, int* err) {
+__global__ void __launch_bounds__(kFieldThreads) k_f_xc(const double* rho, int64_t total,
+                                                        double* vxc, double2* work,
+                                                        double* part, int* err) {
   chain_wait();
   __shared__ double sm[kFieldThreads];
   double s_ex = 0.0, s_vx = 0.0;
@@ -120,7 +120,7 @@ __device__ __forceinline__ int64_t line_base(const Box3& b, int axis, int64_t L,
 }
 
 template <int SIGN>
-__global__ void __launch_bounds__(kFieldThreads) k_f_lines(double2* __restrict__ data, Box3 b, int axis, FftPlan plan,
+__global__ void __launch_bounds__(kFieldThreads) k_f_lines(double2* data, Box3 b, int axis, FftPlan plan,
                                                            const double2* __restrict__ twg) {
   chain_wait();
   extern __shared__ double2 fsm[];
@@ -166,7 +166,7 @@ struct Recip {
   double b[3][3];  // b[i][j]: Cartesian component i of reciprocal vector j (Bohr^-1)
 };
 
-__global__ void __launch_bounds__(kFieldThreads) k_f_poisson(double2* __restrict__ work, Box3 bx, Recip rc,
+__global__ void __launch_bounds__(kFieldThreads) k_f_poisson(double2* work, Box3 bx, Recip rc,
                                                              double inv_n) {
   chain_wait();
   for (int64_t p = blockIdx.x * (int64_t)kFieldThreads + threadIdx.x; p < bx.total;
@@ -190,11 +190,11 @@ __global__ void __launch_bounds__(kFieldThreads) k_f_poisson(double2* __restrict
   }
 }
 
-__global__ void __launch_bounds__(kFieldThreads) k_f_collect(const double2* __restrict__ work,
-                                                             const double* __restrict__ rho,
-                                                             const double* __restrict__ vxc, int64_t total,
-                                                             double* __restrict__ v_h, double* __restrict__ v_hxc,
-                                                             double* __restrict__ part) {
+__global__ void __launch_bounds__(kFieldThreads) k_f_collect(const double2* work,
+                                                             const double* rho,
+                                                             const double* vxc, int64_t total,
+                                                             double* v_h, double* v_hxc,
+                                                             double* part) {
   chain_wait();
   __shared__ double sm[kFieldThreads];
   double s_eh = 0.0;
@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(kFieldThreads) k_f_collect(const double2* __re
 
 // The block sums in a fixed tree: thread t adds blocks t, t + 256, ... in order.  (One thread
 // walking the 592 x 3 sums took 52 us of the 460 us Si64 field step, a chain of dependent loads.)
-__global__ void __launch_bounds__(kFieldThreads) k_f_energies(const double* __restrict__ part, int blocks, double dv,
-                                                              double* __restrict__ out) {
+__global__ void __launch_bounds__(kFieldThreads) k_f_energies(const double* part, int blocks, double dv,
+                                                              double* out) {
   chain_wait();
   __shared__ double sm[kFieldThreads];
   double s[3] = {0.0, 0.0, 0.0};
@@ -229,26 +229,26 @@ __global__ void __launch_bounds__(kFieldThreads) k_f_energies(const double* __re
 // Density sphere transforms of the mixer (crates/dft-engine/src/refscf/density.rs:
 // 173-237): forward picks FFT(rho)/N on the half-sphere indices; inverse forms
 // 2 Re(sum_half c_G e^{iGr}) - Re c_0 from the half-sphere coefficients alone.
-__global__ void k_f_load_real(const double* __restrict__ rho, int64_t total, double2* __restrict__ work) {
+__global__ void k_f_load_real(const double* rho, int64_t total, double2* work) {
   chain_wait();
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < total; p += (int64_t)gridDim.x * blockDim.x)
     work[p] = make_double2(rho[p], 0.0);
 }
-__global__ void k_f_zero(double2* __restrict__ work, int64_t total) {
+__global__ void k_f_zero(double2* work, int64_t total) {
   chain_wait();
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < total; p += (int64_t)gridDim.x * blockDim.x)
     work[p] = make_double2(0.0, 0.0);
 }
-__global__ void k_f_pick(const double2* __restrict__ work, const int64_t* __restrict__ idx, int64_t n, double inv_n,
-                         double2* __restrict__ out) {
+__global__ void k_f_pick(const double2* work, const int64_t* __restrict__ idx, int64_t n, double inv_n,
+                         double2* out) {
   chain_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const double2 z = work[idx[i]];
     out[i] = make_double2(z.x * inv_n, z.y * inv_n);
   }
 }
-__global__ void k_f_place(const double2* __restrict__ c, const int64_t* __restrict__ idx, int64_t n,
-                          double2* __restrict__ work, int* err) {
+__global__ void k_f_place(const double2* c, const int64_t* __restrict__ idx, int64_t n,
+                          double2* work, int* err) {
   chain_wait();
   bool bad = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -258,8 +258,8 @@ __global__ void k_f_place(const double2* __restrict__ c, const int64_t* __restri
   }
   if (bad) atomicOr(err, 1);
 }
-__global__ void k_f_half_real(const double2* __restrict__ work, const double2* __restrict__ c, int64_t i0,
-                              int64_t total, double* __restrict__ rho) {
+__global__ void k_f_half_real(const double2* work, const double2* c, int64_t i0,
+                              int64_t total, double* rho) {
   chain_wait();
   const double g0 = i0 >= 0 ? c[i0].x : 0.0;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < total; p += (int64_t)gridDim.x * blockDim.x)

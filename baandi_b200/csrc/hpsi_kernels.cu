@@ -479,8 +479,8 @@ __global__ void k_couple(const NlDev* __restrict__ nls, int nproj, int ksplit, B
   const int cols = resolve(b.a[blockIdx.z]).cols;
   const int atom = blockIdx.x, c = blockIdx.y;
   if (c >= cols) return;
-  const T* __restrict__ part = reinterpret_cast<const T*>(nl.part);
-  T* __restrict__ wd = reinterpret_cast<T*>(nl.wd);
+  const T* part = reinterpret_cast<const T*>(nl.part);
+  T* wd = reinterpret_cast<T*>(nl.wd);
   const int* __restrict__ atom_off = nl.atom_off;
   const int* __restrict__ d_off = nl.d_off;
   const double* __restrict__ d = nl.d;
@@ -540,8 +540,8 @@ constexpr int density_blocks_per_sm() {
 // and one block of eight warps: 11.0 ms for the 480 Si216 bands.)
 template <int N>
 __global__ void __launch_bounds__(planes_threads<N, double2>(), density_blocks_per_sm<N>())
-    k_density_planes_fast(const OpTables* __restrict__ tabs, BoxGeo g, Batch b, int gamma, const double* __restrict__ w,
-                          int wstride, int unit0, double* __restrict__ part) {
+    k_density_planes_fast(const OpTables* __restrict__ tabs, BoxGeo g, Batch b, int gamma, const double* w,
+                          int wstride, int unit0, double* part) {
   chain_wait();
   using Pl = fast::Plan<N>;
   static_assert(Pl::nst == 2, "two-stage plans");
@@ -598,8 +598,8 @@ __global__ void __launch_bounds__(planes_threads<N, double2>(), density_blocks_p
 
 // The same for planes outside fft_any.cuh.
 __global__ void __launch_bounds__(256, 1) k_density_planes(const OpTables* __restrict__ tabs, BoxGeo g, Batch b,
-                                                        int gamma, const double* __restrict__ w, int wstride,
-                                                        int unit0, double* __restrict__ part) {
+                                                        int gamma, const double* w, int wstride,
+                                                        int unit0, double* part) {
   chain_wait();
   const OpTables& t = tabs[blockIdx.z];
   const CallArgs& a = b.a[blockIdx.z];
@@ -636,8 +636,8 @@ __global__ void __launch_bounds__(256, 1) k_density_planes(const OpTables* __res
 // ksum[k][q] (first: =, else +=) sum_c part[k][c][q], units in order (q in the partial slices'
 // z, y, x order), divided by the volume after the last group; blockIdx.y = k, so the k points'
 // chains run side by side.
-__global__ void k_density_sum_chunks(const double* __restrict__ part, int chunks, int64_t total, double volume,
-                                     int first, int last, double* __restrict__ ksum) {
+__global__ void k_density_sum_chunks(const double* part, int chunks, int64_t total, double volume,
+                                     int first, int last, double* ksum) {
   chain_wait();
   const int k = blockIdx.y;
   const double* pk = part + (int64_t)k * chunks * total;
@@ -651,8 +651,8 @@ __global__ void k_density_sum_chunks(const double* __restrict__ part, int chunks
 
 // out[x][y][z] (= or +=) sum_k ksum[k][z][y n0 + x], k points added one after the other
 // (the arithmetic of one call per k point accumulating into out).
-__global__ void k_density_sum_k(const double* __restrict__ ksum, int nk, int n0, int n1, int n2, int accumulate,
-                                double* __restrict__ out) {
+__global__ void k_density_sum_k(const double* ksum, int nk, int n0, int n1, int n2, int accumulate,
+                                double* out) {
   chain_wait();
   const int64_t pts = (int64_t)n0 * n1, total = pts * n2;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
@@ -1023,7 +1023,7 @@ int configure_kernels(size_t plane_smem, size_t stick_smem) {
 // Descriptors of the tensor-core nonlocal products of every operator of a batch:
 // [k] P^H x into the projection buffer, [nk + k] y += P wd, P from the operator's
 // split panels.  One thread per operator.
-__global__ void k_nl_tc_descs(const NlDev* __restrict__ nls, int nproj, Batch b, tc::ZDesc* __restrict__ out) {
+__global__ void k_nl_tc_descs(const NlDev* __restrict__ nls, int nproj, Batch b, tc::ZDesc* out) {
   chain_wait();
   const int k = threadIdx.x;
   if (k >= b.nk) return;
@@ -1072,7 +1072,7 @@ int ensure_nonlocal_tc(TcNl* t, int nk, int nproj, int max_cols, int max_rows) {
 
 // Descriptors of the FP64 residue products of every operator of a batch: [k] P^H x into the
 // projection buffer, [nk + k] y += P wd.  One thread per operator.
-__global__ void k_nl_rns_descs(const NlDev* __restrict__ nls, int nproj, Batch b, rns::Desc* __restrict__ out) {
+__global__ void k_nl_rns_descs(const NlDev* __restrict__ nls, int nproj, Batch b, rns::Desc* out) {
   chain_wait();
   const int k = threadIdx.x;
   if (k >= b.nk) return;

@@ -580,7 +580,7 @@ __device__ bool eigen(const Bufs<D>& b, int cap, int m, double* red, int* sh) {
 // runs over the column tiles, so the blocks that read one 64-row slice of the tall A
 // launch together and share it in L2.
 template <class D>
-__global__ void __launch_bounds__(256, 2) k_dv_nn(const Bufs<D>* __restrict__ bufs, const NN<D>* __restrict__ desc,
+__global__ void __launch_bounds__(256, 2) k_dv_nn(const Bufs<D>* bufs, const NN<D>* desc,
                                                   int nk, int residues) {
   chain_wait();
   const int z = blockIdx.z, k = z % nk;
@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(256, 2) k_dv_nn(const Bufs<D>* __restrict__ bu
 // Split-K partial Gram products: part[slot][s][j][i] = sum over row slice s of
 // conj(A[r][i]) B[r][j]; blockIdx.z = (slot * nk + k) * ks + s.
 template <class D>
-__global__ void __launch_bounds__(256, 2) k_dv_tn(const Bufs<D>* __restrict__ bufs, const TN<D>* __restrict__ desc, int nk,
+__global__ void __launch_bounds__(256, 2) k_dv_tn(const Bufs<D>* bufs, const TN<D>* desc, int nk,
                                               int ks, int64_t slot_elems, int residues) {
   chain_wait();
   const int zz = blockIdx.z / ks, sidx = blockIdx.z % ks;
@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(256, 2) k_dv_tn(const Bufs<D>* __restrict__ bu
 
 // G[i + j ldg] = sum_s part[slot][s][j][i] in slice order.
 template <class D>
-__global__ void k_dv_tn_sum(const Bufs<D>* __restrict__ bufs, const TN<D>* __restrict__ desc, int nk, int ks,
+__global__ void k_dv_tn_sum(const Bufs<D>* bufs, const TN<D>* desc, int nk, int ks,
                             int64_t slot_elems, int residues) {
   chain_wait();
   const int zz = blockIdx.z, slot = zz / nk, k = zz % nk;
@@ -635,7 +635,7 @@ __global__ void k_dv_tn_sum(const Bufs<D>* __restrict__ bufs, const TN<D>* __res
 // descriptor reads are paid for once per kCopyUnroll x 256 rows.
 constexpr int kCopyUnroll = 4;
 template <class D>
-__global__ void k_dv_copy(const Bufs<D>* __restrict__ bufs, const CP<D>* __restrict__ desc, int nk) {
+__global__ void k_dv_copy(const Bufs<D>* bufs, const CP<D>* desc, int nk) {
   chain_wait();
   const int z = blockIdx.z, k = z % nk;
   const CP<D> d = desc[z];
@@ -679,9 +679,9 @@ __global__ void __launch_bounds__(128) k_dv_dense(const D* const* __restrict__ H
 // Corrections of the active bands of every running k point (correction_column with the
 // solver's preconditioner), norms[j] = |Er[:, j]|^2.
 template <class D>
-__global__ void __launch_bounds__(256) k_dv_corrections(const Bufs<D>* __restrict__ bufs, const Ctl* __restrict__ ctl,
-                                                        const Opts* __restrict__ opts,
-                                                        const __nv_bfloat16* __restrict__ net) {
+__global__ void __launch_bounds__(256) k_dv_corrections(const Bufs<D>* bufs, const Ctl* ctl,
+                                                        const Opts* opts,
+                                                        const __nv_bfloat16* net) {
   chain_wait();
   __shared__ double red[256];
   __shared__ float wnet[learned::kParams];
@@ -710,8 +710,8 @@ __global__ void __launch_bounds__(256) k_dv_corrections(const Bufs<D>* __restric
 // Tensor-core descriptors of the products marked prec = 1 (complex blocks): one thread per
 // (slot, k point); the others get empty descriptors.
 template <class D>
-__global__ void k_dv_tc_descs(const Bufs<D>* __restrict__ bufs, const NN<D>* __restrict__ nn, int n_nn,
-                              const TN<D>* __restrict__ tn, int n_tn, int nk, tc::ZDesc* out_nn, tc::ZDesc* out_tn) {
+__global__ void k_dv_tc_descs(const Bufs<D>* bufs, const NN<D>* nn, int n_nn,
+                              const TN<D>* tn, int n_tn, int nk, tc::ZDesc* out_nn, tc::ZDesc* out_tn) {
   chain_wait();
   const int z = blockIdx.x * blockDim.x + threadIdx.x;
   const tc::ZDesc empty{nullptr, nullptr, nullptr, 1, 1, 1, 0, 0, 0, tc::kStore};
@@ -737,8 +737,8 @@ __global__ void k_dv_tc_descs(const Bufs<D>* __restrict__ bufs, const NN<D>* __r
 // Residue-product descriptors of the FP64 products that pay there (complex blocks): one
 // thread per (slot, k point); the others get empty descriptors.
 template <class D>
-__global__ void k_dv_rns_descs(const Bufs<D>* __restrict__ bufs, const NN<D>* __restrict__ nn, int n_nn,
-                               const TN<D>* __restrict__ tn, int n_tn, int nk, rns::Desc* out) {
+__global__ void k_dv_rns_descs(const Bufs<D>* bufs, const NN<D>* nn, int n_nn,
+                               const TN<D>* tn, int n_tn, int nk, rns::Desc* out) {
   chain_wait();
   const int z = blockIdx.x * blockDim.x + threadIdx.x;
   rns::Desc o{nullptr, nullptr, nullptr, 1, 1, 1, 0, 0, 0, rns::kStore};
@@ -795,9 +795,9 @@ enum Phase : int {
 constexpr int kNnSlots = 2, kTnSlots = 2, kCpSlots = 3;
 
 template <class D>
-__global__ void __launch_bounds__(kCtlThreads, 1) k_dv_ctl(int phase, Bufs<D>* __restrict__ bufs, Ctl* ctl,
+__global__ void __launch_bounds__(kCtlThreads, 1) k_dv_ctl(int phase, Bufs<D>* bufs, Ctl* ctl,
                                                         NN<D>* nn, TN<D>* tn, CP<D>* cp, DynCols* dyn,
-                                                        const Opts* __restrict__ opts, int nk, int gamma) {
+                                                        const Opts* opts, int nk, int gamma) {
   chain_wait();
   using X = Cx<D>;
   const Opts o = *opts;
@@ -1338,7 +1338,7 @@ struct IoPtrs {
 // Zero S, H_r, L, C of every k point and copy its start block and diagonal from device
 // pointers: one launch instead of six stream operations per k point.  blockIdx.y = k.
 template <class D>
-__global__ void k_dv_init(const Bufs<D>* __restrict__ bufs, const IoPtrs* __restrict__ io, int n, int cap) {
+__global__ void k_dv_init(const Bufs<D>* bufs, const IoPtrs* io, int n, int cap) {
   chain_wait();
   const int k = blockIdx.y;
   const Bufs<D>& b = bufs[k];
@@ -1366,8 +1366,8 @@ __global__ void k_dv_init(const Bufs<D>* __restrict__ bufs, const IoPtrs* __rest
 // convergence flags and the operator's error word gathered for one read by the host
 // (out: nk n values, then nk n flags and nk error words as doubles).  blockIdx.y = k.
 template <class D>
-__global__ void k_dv_out(const Bufs<D>* __restrict__ bufs, const IoPtrs* __restrict__ io, int n, int nk,
-                         double* __restrict__ out) {
+__global__ void k_dv_out(const Bufs<D>* bufs, const IoPtrs* io, int n, int nk,
+                         double* out) {
   chain_wait();
   const int k = blockIdx.y;
   const Bufs<D>& b = bufs[k];

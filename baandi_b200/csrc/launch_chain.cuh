@@ -3,7 +3,13 @@
 // ramp of its first blocks then overlap the predecessor's tail), and chain_wait at the top
 // of every such kernel holds them until the predecessor has finished and its writes are
 // visible.  Every block calls it first, also where it returns at once: a kernel that could
-// finish before its own predecessor would release its successor too early.  Measured (chained
+// finish before its own predecessor would release its successor too early.
+//
+// A chained kernel lives while its predecessor still writes, so __restrict__ on one of its
+// parameters is a promise that holds only for tables that no kernel writes (the compiler may
+// read a const __restrict__ buffer through the non-coherent path, and may move any access
+// through a __restrict__ pointer above the wait, which it takes not to touch it).  Buffers that
+// kernels write stay without it; tests/test_launch_chain.py holds the list.  Measured (chained
 // against plain launches): the Si2 Gamma apply's six kernels 40.3 -> 32.5 us, one Si8 k point's
 // 88.1 -> 82.0 us, the Si64 field step's 24 286 -> 244 us, 308 launches of an Si216 eigenproblem
 // 2 ms of 145 ms.

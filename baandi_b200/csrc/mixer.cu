@@ -42,8 +42,8 @@ __device__ __forceinline__ void neu_add(Neu& a, double v) {
   a.s = t;
 }
 
-__global__ void k_mix_diff(const double2* __restrict__ x, const double2* __restrict__ f, double2* prev_x,
-                           double2* prev_f, double2* __restrict__ dx, double2* __restrict__ df, int64_t n, int have_slot) {
+__global__ void k_mix_diff(const double2* x, const double2* f, double2* prev_x,
+                           double2* prev_f, double2* dx, double2* df, int64_t n, int have_slot) {
   chain_wait();
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
     const double2 xv = x[j], fv = f[j];
@@ -59,9 +59,9 @@ __global__ void k_mix_diff(const double2* __restrict__ x, const double2* __restr
 
 // forms[q] for q < p(p+1)/2: <dF_i, dF_j> (i >= j, row-major lower triangle);
 // forms[p(p+1)/2 + i] = <dF_i, F>.  One block per form.
-__global__ void __launch_bounds__(kMixThreads) k_mix_forms(const double2* __restrict__ df, int64_t n, int p,
-                                                           const double2* __restrict__ f,
-                                                           const double* __restrict__ w, double* __restrict__ forms) {
+__global__ void __launch_bounds__(kMixThreads) k_mix_forms(const double2* df, int64_t n, int p,
+                                                           const double2* f,
+                                                           const double* w, double* forms) {
   chain_wait();
   const int q = blockIdx.x;
   const int tri = p * (p + 1) / 2;
@@ -101,8 +101,8 @@ __global__ void __launch_bounds__(kMixThreads) k_mix_forms(const double2* __rest
 // One thread: Jacobi eigen-decomposition of the p x p Gram, rank test, gamma.
 // out[0] = status (0 ok, 1 singular, 2 non-finite), out[1] = lambda_min,
 // out[2] = lambda_max, out[3] = condition.
-__global__ void k_mix_solve(const double* __restrict__ forms, int p, double* __restrict__ gamma,
-                            double* __restrict__ out) {
+__global__ void k_mix_solve(const double* forms, int p, double* gamma,
+                            double* out) {
   chain_wait();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   double A[kMaxHistory][kMaxHistory], Q[kMaxHistory][kMaxHistory];
@@ -179,11 +179,11 @@ __global__ void k_mix_solve(const double* __restrict__ forms, int p, double* __r
   out[0] = 0.0;
 }
 
-__global__ void k_mix_apply(const double2* __restrict__ x, const double2* __restrict__ f,
-                            const double2* __restrict__ dx, const double2* __restrict__ df, int64_t n, int p,
-                            const double* __restrict__ gamma, const int* __restrict__ smooth,
-                            const double* __restrict__ screening, double beta, double2* __restrict__ next,
-                            double2* __restrict__ reduced, int* err) {
+__global__ void k_mix_apply(const double2* x, const double2* f,
+                            const double2* dx, const double2* df, int64_t n, int p,
+                            const double* gamma, const int* __restrict__ smooth,
+                            const double* __restrict__ screening, double beta, double2* next,
+                            double2* reduced, int* err) {
   chain_wait();
   __shared__ double g[kMaxHistory];
   if ((int)threadIdx.x < p) g[threadIdx.x] = gamma[threadIdx.x];

@@ -84,8 +84,8 @@ __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1) k_planes_any(const OpT
 template <int W>
 __global__ void __launch_bounds__(32 * W, W == 8 ? 2 : 1)
     k_density_planes_any(const OpTables* __restrict__ tabs, const __grid_constant__ BoxGeo g,
-                         const __grid_constant__ Batch b, int gamma, const double* __restrict__ w, int wstride,
-                         int unit0, double* __restrict__ part) {
+                         const __grid_constant__ Batch b, int gamma, const double* w, int wstride,
+                         int unit0, double* part) {
   chain_wait();
   const OpTables& t = tabs[blockIdx.z];
   const CallArgs& a = b.a[blockIdx.z];
