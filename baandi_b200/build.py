@@ -40,8 +40,8 @@ def stale() -> bool:
         for f in files:
             if os.path.getmtime(os.path.join(root, f)) > t:
                 return True
-    inc = os.path.join(HERE, "..", "include", "baandi_gpu.h")
-    return os.path.exists(inc) and os.path.getmtime(inc) > t
+    inc = os.path.join(HERE, "..", "include")
+    return os.path.isdir(inc) and any(os.path.getmtime(os.path.join(inc, f)) > t for f in os.listdir(inc))
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

@@ -17,6 +17,7 @@
 #include "gemm_tc.cuh"
 #include "op_internal.h"
 #include "plane_passes.cuh"
+#include "../../include/baandi_gpu_test.h"
 
 namespace bg {
 static thread_local std::string g_error;
@@ -767,6 +768,16 @@ int bg_op_sync(bg_op* op) {
   return check_err(op);
 }
 
+int bg_test_raise_error(bg_op* op, int32_t bits) {
+  if (!op) return fail(nullptr, BG_EINVAL, "null operator");
+  int word = 0;
+  cudaError_t e = cudaStreamSynchronize(op->stream);
+  if (e == cudaSuccess) e = cudaMemcpy(&word, op->t.err, sizeof(int), cudaMemcpyDeviceToHost);
+  word |= bits;
+  if (e == cudaSuccess) e = cudaMemcpy(op->t.err, &word, sizeof(int), cudaMemcpyHostToDevice);
+  return e == cudaSuccess ? BG_OK : cuda_fail(op->ctx, e, "error word");
+}
+
 int bg_op_diagonal(const bg_op* op, double* out) {
   if (!op || !out) return fail(op ? op->ctx : nullptr, BG_EINVAL, "null argument");
   std::copy(op->diag.begin(), op->diag.end(), out);
@@ -1157,7 +1168,7 @@ int bg_kset_set_potential_ptr(bg_kset* ks, const double* v, uint64_t epoch, int3
   if (op0->err_host[0]) {
     cudaMemsetAsync(op0->t.err, 0, sizeof(int), ks->stream);
     cudaStreamSynchronize(ks->stream);
-    return fail(ctx, BG_ENONFINITE, "non-finite potential value");
+    return report_error_bits(ctx, op0->err_host[0]);
   }
   launch_broadcast(op0->vchange, (int64_t)vdoubles, ks->d_vts, n, ks->stream);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
@@ -1481,9 +1492,9 @@ int bg_kset_sync(bg_kset* ks) {
   e = cudaMemcpyAsync(ks->h_errv, ks->d_errv, n * sizeof(int), cudaMemcpyDeviceToHost, ks->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ks->stream);
   if (e != cudaSuccess) return cuda_fail(ks->ctx, e, "k-point set");
-  for (int k = 0; k < n; ++k)
-    if (ks->h_errv[k]) return report_error_bits(ks->ctx, ks->h_errv[k]);
-  return BG_OK;
+  int bits = 0;
+  for (int k = 0; k < n; ++k) bits |= ks->h_errv[k];
+  return report_error_bits(ks->ctx, bits);
 }
 
 int bg_kset_stream(const bg_kset* ks, void** stream) {

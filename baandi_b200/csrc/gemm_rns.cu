@@ -12,12 +12,12 @@
 #include "gemm_rns.cuh"
 
 #include <algorithm>
+#include <vector>
 
 namespace bg {
 namespace rns {
 namespace {
 
-constexpr unsigned kWaitLimit = 1u << 24;
 constexpr int kSms = 148;
 constexpr int kMaxDesc = 128;
 constexpr int kStages = 6;
@@ -155,8 +155,8 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t mbar, uint32_t bytes) {
       : "memory");
 }
 // Bounded wait; gives up early once another role of the block has.
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, volatile int* failed) {
-  for (unsigned i = 0; i < kWaitLimit; ++i) {
+__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, volatile int* failed, unsigned limit) {
+  for (unsigned i = 0; i < limit; ++i) {
     uint32_t ok;
     asm volatile(
         "{\n\t"
@@ -463,15 +463,15 @@ __device__ __forceinline__ void reduce_store(const int (&x)[16], int p, int c16,
 // issues the MMAs (two 128-row halves share each B tile: 64 bytes of L2 traffic per SM and
 // cycle at the full int8 rate, where a single 128-row tile would need 96); the epilogue
 // warps reduce the int32 accumulators modulo p and store bytes.  With trb <= 128 the
-// accumulator is double buffered in tensor memory.  Every wait is bounded; a role that
-// gives up stops the block, which waits (bounded) for its own copies and MMAs, frees its
-// tensor memory and sets the error word.  SHORT: K 121^2 < 2^24 (a cheaper
+// accumulator is double buffered in tensor memory.  Every wait is bounded (the roles' by
+// `limit` tries); a role that gives up stops the block, which waits (bounded by kWaitLimit) for
+// its own copies and MMAs, frees its tensor memory and sets the error word.  SHORT: K 121^2 < 2^24 (a cheaper
 // reduction).  256 x 256 tiles measured 0.94 and 1.38 ms (kTN, kNN at Si216) where 256 x 128
 // double-buffered ones took 1.55 and 1.74 ms; loading the next columns during the reduction
 // took 0.94 and 1.38 to 0.87 and 1.07 ms.
 template <bool SHORT>
 __global__ void __launch_bounds__(kMmaThreads, 1)
-    k_rns_mma(const Desc* __restrict__ descs, int ndesc, Geo g, unsigned char* work, int* err) {
+    k_rns_mma(const Desc* __restrict__ descs, int ndesc, Geo g, unsigned char* work, int* err, unsigned limit) {
   extern __shared__ unsigned char dyn[];
   __shared__ __align__(8) uint64_t full[kStages], empty[kStages], tfull[2], tempty[2];
   __shared__ uint32_t tmem_slot;
@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
           work + g.b_off + it.z * g.b_stride + (((size_t)it.plane * g.nt + it.nt) * g.ktc + it.kb) * bbytes;
       for (int k = 0; k < it.ke - it.kb; ++k, ++t) {
         const int s = t % kStages;
-        if (t >= kStages && !mbar_wait(smem_addr(&empty[s]), (uint32_t)((t / kStages - 1) & 1), failed)) {
+        if (t >= kStages && !mbar_wait(smem_addr(&empty[s]), (uint32_t)((t / kStages - 1) & 1), failed, limit)) {
           s_fail = 1;
           break;
         }
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
       const int buf = n % nbuf, use = n / nbuf;
       const int ncols = min(trb, s_n[it.z] - it.nt * trb);
       const uint32_t id = idesc((ncols + 15) / 16 * 16);
-      if (use > 0 && !mbar_wait(smem_addr(&tempty[buf]), (uint32_t)((use - 1) & 1), failed)) {
+      if (use > 0 && !mbar_wait(smem_addr(&tempty[buf]), (uint32_t)((use - 1) & 1), failed, limit)) {
         s_fail = 1;
         break;
       }
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
       const uint32_t acc = tmem + (uint32_t)buf * 2 * acc_cols;
       for (int k = 0; k < it.ke - it.kb; ++k, ++t) {
         const int s = t % kStages;
-        if (!mbar_wait(smem_addr(&full[s]), (uint32_t)((t / kStages) & 1), failed)) {
+        if (!mbar_wait(smem_addr(&full[s]), (uint32_t)((t / kStages) & 1), failed, limit)) {
           s_fail = 1;
           ok = false;
           break;
@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
       const int buf = n % nbuf, use = n / nbuf;
       ++n;
       bool ok = true;
-      if (lane == 0) ok = mbar_wait(smem_addr(&tfull[buf]), (uint32_t)(use & 1), failed);
+      if (lane == 0) ok = mbar_wait(smem_addr(&tfull[buf]), (uint32_t)(use & 1), failed, limit);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) {
         if (lane == 0) s_fail = 1;
@@ -659,10 +659,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
     __shared__ int s_none;
     if (tid == 0) {
       s_none = 0;
-      for (int t = s_consumed; t < s_issued; ++t) mbar_wait(smem_addr(&full[t % kStages]), (uint32_t)((t / kStages) & 1), &s_none);
+      for (int t = s_consumed; t < s_issued; ++t) mbar_wait(smem_addr(&full[t % kStages]), (uint32_t)((t / kStages) & 1), &s_none, kWaitLimit);
       if (s_consumed > 0) {
         const int t = s_consumed - 1;
-        mbar_wait(smem_addr(&empty[t % kStages]), (uint32_t)((t / kStages) & 1), &s_none);
+        mbar_wait(smem_addr(&empty[t % kStages]), (uint32_t)((t / kStages) & 1), &s_none, kWaitLimit);
       }
       atomicOr(err, kErrBit);
     }
@@ -836,7 +836,7 @@ cudaError_t prepare() {
 }
 
 int launch_product(int mode, const Desc* d_desc, int ndesc, int max_m, int max_n, int max_k, bool a_presplit,
-                   void* work, size_t work_bytes, int* err, cudaStream_t s) {
+                   void* work, size_t work_bytes, int* err, cudaStream_t s, unsigned wait_limit) {
   if (ndesc == 0 || max_m <= 0 || max_n <= 0 || max_k <= 0) return 0;
   const Geo g = carve(mode, ndesc, max_m, max_n, max_k, a_presplit, work_bytes);
   unsigned char* w = static_cast<unsigned char*>(work);
@@ -858,9 +858,9 @@ int launch_product(int mode, const Desc* d_desc, int ndesc, int max_m, int max_n
   }
   const int kper = (int)std::min<int64_t>(max_k, (int64_t)kTileK * ((g.ktc + g.ksplit - 1) / g.ksplit));
   if ((int64_t)kper * 121 * 121 < (1 << 24))
-    k_rns_mma<true><<<kSms, kMmaThreads, mma_smem(g.trb), s>>>(d_desc, ndesc, g, w, err);
+    k_rns_mma<true><<<kSms, kMmaThreads, mma_smem(g.trb), s>>>(d_desc, ndesc, g, w, err, wait_limit);
   else
-    k_rns_mma<false><<<kSms, kMmaThreads, mma_smem(g.trb), s>>>(d_desc, ndesc, g, w, err);
+    k_rns_mma<false><<<kSms, kMmaThreads, mma_smem(g.trb), s>>>(d_desc, ndesc, g, w, err, wait_limit);
   const int64_t blocks = (int64_t)((max_m + 127) / 128) * ((max_n + 3) / 4);
   const dim3 jg((unsigned)std::min<int64_t>(blocks, std::max(148, kSms * 24 / ndesc)), ndesc);
   if (mode == kTN)
@@ -889,40 +889,60 @@ cudaError_t split_a(int mode, const double2* A, int64_t lda, int M, int K, unsig
 }  // namespace rns
 }  // namespace bg
 
-// ------------------------------------------------------------------ test entry
+// ------------------------------------------------------------------ test entries
+#include "../../include/baandi_gpu_test.h"
 #include "op_internal.h"
 
 using namespace bg;
 
-// One product of device matrices (column-major interleaved complex, as bg_zgemm_bf16x3), for
-// the tests of the tile edges: presplit takes A through split_a.  Returns a BG_ status.
-extern "C" int bg_test_residue_product(int32_t mode, int64_t m, int64_t n, int64_t k, const double* a, int64_t lda,
-                                       const double* b, int64_t ldb, double* c, int64_t ldc, int32_t op,
-                                       int32_t presplit) {
+extern "C" int bg_test_residue_products(int32_t mode, int32_t count, const int64_t* shapes, const double* const* a,
+                                        const int64_t* lda, const double* const* b, const int64_t* ldb,
+                                        double* const* c, const int64_t* ldc, int32_t op, int32_t presplit,
+                                        const int64_t* bounds, int64_t wait_limit) {
   using namespace bg::rns;
-  Desc d{reinterpret_cast<const double2*>(a), reinterpret_cast<const double2*>(b), reinterpret_cast<double2*>(c), lda,
-         ldb, ldc, (int)m, (int)n, (int)k, op};
-  DevBuf desc, panel, scale, err, work;
+  if (count < 1 || count > kMaxDesc || !shapes || !a || !b || !c || !lda || !ldb || !ldc) return BG_EINVAL;
+  int64_t top[3] = {0, 0, 0};
+  for (int z = 0; z < count; ++z)
+    for (int i = 0; i < 3; ++i) top[i] = std::max(top[i], shapes[3 * z + i]);
+  std::vector<Desc> h(count);
+  std::vector<DevBuf> panel(count), scale(count);
+  DevBuf desc, err, work;
   auto alloc = [](DevBuf* x, size_t bytes) { return cudaMalloc(&x->p, bytes) == cudaSuccess; };
-  const size_t wb = workspace_bytes(mode, 1, (int)m, (int)n, (int)k, presplit != 0);
-  if (prepare() != cudaSuccess || !alloc(&desc, sizeof d) || !alloc(&err, sizeof(int)) || !alloc(&work, wb) ||
-      !alloc(&scale, 2 * sizeof(double) * m) || (presplit && !alloc(&panel, a_panel_bytes(m, k))))
+  size_t wb = 0;
+  if (bounds)
+    wb = workspace_bytes(mode, count, (int)bounds[0], (int)bounds[1], (int)bounds[2], presplit != 0);
+  else
+    wb = workspace_bytes(mode, count, (int)top[0], (int)top[1], (int)top[2], presplit != 0);
+  if (prepare() != cudaSuccess || !alloc(&desc, sizeof(Desc) * count) || !alloc(&err, sizeof(int)) || !alloc(&work, wb))
     return BG_ENOMEM;
-  if (presplit) {
-    double* s = static_cast<double*>(scale.p);
-    if (split_a(mode, d.A, lda, (int)m, (int)k, static_cast<unsigned char*>(panel.p), s, s + m, nullptr) != cudaSuccess)
+  for (int z = 0; z < count; ++z) {
+    const int64_t m = shapes[3 * z], n = shapes[3 * z + 1], k = shapes[3 * z + 2];
+    h[z] = Desc{reinterpret_cast<const double2*>(a[z]), reinterpret_cast<const double2*>(b[z]),
+                reinterpret_cast<double2*>(c[z]), lda[z], ldb[z], ldc[z], (int)m, (int)n, (int)k, op};
+    if (!presplit || m <= 0 || k <= 0) continue;
+    if (!alloc(&scale[z], 2 * sizeof(double) * m) || !alloc(&panel[z], a_panel_bytes(m, k))) return BG_ENOMEM;
+    double* s = static_cast<double*>(scale[z].p);
+    if (split_a(mode, h[z].A, lda[z], (int)m, (int)k, static_cast<unsigned char*>(panel[z].p), s, s + m, nullptr) !=
+        cudaSuccess)
       return BG_EDEVICE;
-    d.a_panel = static_cast<const unsigned char*>(panel.p);
-    d.a_inv = s + m;
-    d.a_kt = k_tiles(k);
+    h[z].a_panel = static_cast<const unsigned char*>(panel[z].p);
+    h[z].a_inv = s + m;
+    h[z].a_kt = k_tiles(k);
   }
   int word = 0;
   if (cudaMemset(err.p, 0, sizeof(int)) != cudaSuccess ||
-      cudaMemcpy(desc.p, &d, sizeof d, cudaMemcpyHostToDevice) != cudaSuccess)
+      cudaMemcpy(desc.p, h.data(), sizeof(Desc) * count, cudaMemcpyHostToDevice) != cudaSuccess)
     return BG_EDEVICE;
-  launch_product(mode, static_cast<Desc*>(desc.p), 1, (int)m, (int)n, (int)k, presplit != 0, work.p, wb,
-                 static_cast<int*>(err.p), nullptr);
+  launch_product(mode, static_cast<Desc*>(desc.p), count, (int)top[0], (int)top[1], (int)top[2], presplit != 0, work.p,
+                 wb, static_cast<int*>(err.p), nullptr, wait_limit < 0 ? kWaitLimit : (unsigned)wait_limit);
   if (cudaGetLastError() != cudaSuccess || cudaMemcpy(&word, err.p, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
     return BG_EDEVICE;
   return word ? BG_ETIMEOUT : BG_OK;
+}
+
+extern "C" int bg_test_residue_product(int32_t mode, int64_t m, int64_t n, int64_t k, const double* a, int64_t lda,
+                                       const double* b, int64_t ldb, double* c, int64_t ldc, int32_t op,
+                                       int32_t presplit) {
+  const int64_t shape[3] = {m, n, k};
+  return bg_test_residue_products(mode, 1, shape, &a, &lda, &b, &ldb, &c, &ldc, op, presplit, nullptr, -1);
 }

@@ -56,6 +56,7 @@ constexpr int kTileK = 64;    // K values per tile
 constexpr int kTileN = 256;   // B rows per tile at most
 constexpr int kMaxK = 131072; // int32 accumulation: K 121^2 < 2^31 per split
 constexpr int kErrBit = 4;    // error-word bit of a bounded wait that gave up
+constexpr unsigned kWaitLimit = 1u << 24;  // tries of a pipeline wait
 
 // One product (device pointers; M = 0 marks an empty slot).
 struct Desc {
@@ -98,9 +99,9 @@ size_t workspace_bytes(int mode, int ndesc, int max_m, int max_n, int max_k, boo
 // descriptor names its A panels.  work: work_bytes at least workspace_bytes of these
 // bounds or of larger ones (fewer K splits are used where the splits of the smaller
 // product would need more).  err: device word, kErrBit set when a
-// bounded wait gives up.  Returns the number of launches.
+// bounded wait gives up (after wait_limit tries).  Returns the number of launches.
 int launch_product(int mode, const Desc* d_desc, int ndesc, int max_m, int max_n, int max_k, bool a_presplit,
-                   void* work, size_t work_bytes, int* err, cudaStream_t s);
+                   void* work, size_t work_bytes, int* err, cudaStream_t s, unsigned wait_limit = kWaitLimit);
 
 // Panels (a_panel_bytes(M, K)) and inverse scales (M doubles) of the A operand of a `mode`
 // product (kTN: K x M, kNN: M x K, ld lda); scale: scratch of M doubles.

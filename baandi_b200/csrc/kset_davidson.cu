@@ -1451,7 +1451,9 @@ class KsetSolver {
   }
   int run(const double* const* start, const double* const* diagonal, int32_t ptr_kind, double* const* values,
           double* const* vectors, int32_t* const* converged, bg_davidson_stats* stats,
-          const double* const* start_hx = nullptr, double* const* vectors_hx = nullptr);
+          const double* const* start_hx = nullptr, double* const* vectors_hx = nullptr) {
+    return settle(solve(start, diagonal, ptr_kind, values, vectors, converged, stats, start_hx, vectors_hx));
+  }
   const std::string& error() const { return err_; }
   int64_t launches() const { return launches_; }
 
@@ -1676,6 +1678,46 @@ class KsetSolver {
     return l;
   }
   int prepare();
+  int solve(const double* const* start, const double* const* diagonal, int32_t ptr_kind, double* const* values,
+            double* const* vectors, int32_t* const* converged, bg_davidson_stats* stats,
+            const double* const* start_hx, double* const* vectors_hx);
+  // The status of a solve that ended with `rc`, from the device error words.  A product whose
+  // pipeline wait gave up leaves wrong values, so it outranks the numerical failure (a dependent
+  // basis, say) that they lead to; its bits are cleared, so no later call reports them.
+  int settle(int rc) {
+    if (rc == BG_EDEVICE || rc == BG_ENOMEM || !prepared_) return rc;
+    bool late = false;
+    int bad = -1;
+    std::vector<int*> words;
+    for (int k = 0; k < nk_; ++k) words.push_back(ks_->ops[k]->t.err);
+    if (tc_ready_) words.push_back(tc_err_);
+    if (tcnl_.err) words.push_back(tcnl_.err);
+    for (int i = 0; i < (int)words.size(); ++i) {
+      // a solve that ended well has brought the operators' words back with its eigenvalues
+      int w = 0, r;
+      if (rc == BG_OK && i < nk_)
+        w = (int)h_out_[2 * (size_t)nk_ * o_.n + i];
+      else if (rc == BG_OK && !o_.tensor)
+        break;
+      else if ((r = cuda(cudaMemcpy(&w, words[i], sizeof(int), cudaMemcpyDeviceToHost), "error word")))
+        return r;
+      const int gave_up = i < nk_ ? (w & rns::kErrBit) : w;
+      late = late || gave_up;
+      if (i < nk_ && rc == BG_OK && (w & ~rns::kErrBit) && bad < 0) bad = i;
+      const int keep = i < nk_ && i != bad ? (w & ~rns::kErrBit) : 0;
+      if (keep != w && (r = cuda(cudaMemcpy(words[i], &keep, sizeof(int), cudaMemcpyHostToDevice), "error word")))
+        return r;
+    }
+    if (late) {
+      err_ = "a tensor-core product's pipeline wait gave up";
+      return BG_ETIMEOUT;
+    }
+    if (bad >= 0) {
+      err_ = "non-finite block in a Davidson apply (k point " + std::to_string(bad) + ")";
+      return BG_ENONFINITE;
+    }
+    return rc;
+  }
   int poll(bool* all_done) {
     int rc = cuda(cudaMemcpyAsync(h_ctl_, d_ctl_, sizeof(Ctl) * nk_, cudaMemcpyDeviceToHost, s_), "poll");
     if (!rc) rc = cuda(cudaStreamSynchronize(s_), "Davidson iteration");
@@ -1781,9 +1823,9 @@ int KsetSolver<T>::prepare() {
 }
 
 template <class T>
-int KsetSolver<T>::run(const double* const* start, const double* const* diagonal, int32_t ptr_kind,
-                       double* const* values, double* const* vectors, int32_t* const* converged,
-                       bg_davidson_stats* stats, const double* const* start_hx, double* const* vectors_hx) {
+int KsetSolver<T>::solve(const double* const* start, const double* const* diagonal, int32_t ptr_kind,
+                         double* const* values, double* const* vectors, int32_t* const* converged,
+                         bg_davidson_stats* stats, const double* const* start_hx, double* const* vectors_hx) {
   const int n = o_.n, cap = o_.cap;
   int rc;
   const bool kept = start_hx != nullptr && ptr_kind == BG_PTR_DEVICE;
@@ -1904,35 +1946,6 @@ int KsetSolver<T>::run(const double* const* start, const double* const* diagonal
     st.dropped = c.dropped;
     st.fallbacks = c.fallbacks;
     if (stats) stats[k] = st;
-  }
-  // the tensor-core products' pipelines (bounded waits) must not have given up
-  if (o_.tensor && tc_ready_) {
-    int words[2] = {0, 0};
-    if ((rc = cuda(cudaMemcpy(&words[0], tc_err_, sizeof(int), cudaMemcpyDeviceToHost), "tensor error word")))
-      return rc;
-    if (tcnl_.err && (rc = cuda(cudaMemcpy(&words[1], tcnl_.err, sizeof(int), cudaMemcpyDeviceToHost), "tensor error word")))
-      return rc;
-    if (words[0] || words[1]) {
-      cudaMemset(tc_err_, 0, sizeof(int));
-      if (tcnl_.err) cudaMemset(tcnl_.err, 0, sizeof(int));
-      err_ = "a tensor-core product's pipeline wait gave up";
-      return BG_ETIMEOUT;
-    }
-  }
-  // a residue product's pipeline wait gave up, or a non-finite block met by the applies
-  for (int k = 0; k < nk_; ++k) {
-    if ((int)h_out_[2 * (size_t)nk_ * n + k] & rns::kErrBit) {
-      cudaMemsetAsync(ks_->ops[k]->t.err, 0, sizeof(int), s_);
-      cudaStreamSynchronize(s_);
-      err_ = "a tensor-core product's pipeline wait gave up";
-      return BG_ETIMEOUT;
-    }
-    if (h_out_[2 * (size_t)nk_ * n + k] != 0.0) {
-      cudaMemsetAsync(ks_->ops[k]->t.err, 0, sizeof(int), s_);
-      cudaStreamSynchronize(s_);
-      err_ = "non-finite block in a Davidson apply (k point " + std::to_string(k) + ")";
-      return BG_ENONFINITE;
-    }
   }
   return BG_OK;
 }

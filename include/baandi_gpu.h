@@ -116,7 +116,8 @@ int bg_op_set_potential(bg_op* op, const double* v_grid, uint64_t epoch);
  * columns, the Gamma operator real ORC columns.  ptr_kind BG_PTR_HOST: synchronous;
  * a non-finite x returns BG_ENONFINITE (y is then unspecified).  BG_PTR_DEVICE:
  * enqueued on the operator's stream, a non-finite x is reported by bg_op_sync; x must
- * not alias y. */
+ * not alias y.  Large FP64 products run on pipelines with bounded waits: one that gives
+ * up is reported the same way as BG_ETIMEOUT (before a non-finite x; y is unspecified). */
 int bg_op_apply_block(bg_op* op, const double* x, double* y, int64_t rows, int64_t cols,
                       int32_t ptr_kind, int32_t precision);
 
@@ -132,7 +133,8 @@ int bg_op_stream(const bg_op* op, void** stream);
 /* Use the caller's stream (cudaStream_t, e.g. a torch stream) for BG_PTR_DEVICE work. */
 int bg_op_set_stream(bg_op* op, void* stream);
 /* Wait for the operator's stream and report a device error recorded by earlier
- * BG_PTR_DEVICE applies (BG_ENONFINITE for a non-finite input column). */
+ * BG_PTR_DEVICE applies (BG_ENONFINITE for a non-finite input column, BG_ETIMEOUT for a
+ * pipeline wait that gave up).  Reported once. */
 int bg_op_sync(bg_op* op);
 /* Count of this library's kernel launches issued by the operator so far. */
 int bg_op_launches(const bg_op* op, int64_t* launches);
