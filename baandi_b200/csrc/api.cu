@@ -48,6 +48,32 @@ int report_error_bits(bg_ctx* ctx, int bits) {
 }
 }  // namespace bg
 
+int DensitySlices::fit(size_t slice, int units, cudaStream_t s) {
+  const size_t bytes = slice * sizeof(double), most = std::max<size_t>(1, budget / bytes);
+  const size_t want = std::min<size_t>((size_t)units, most);
+  size_t have = doubles / slice;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (have < want && cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone) {
+    size_t free = 0, total = 0;
+    size_t n = std::max(want, std::min(2 * have, most));
+    if (cudaMemGetInfo(&free, &total) == cudaSuccess) n = std::min(n, std::max<size_t>(1, free / 4 / bytes));
+    for (; n > have; n /= 2) {
+      auto b = std::make_unique<DevBuf>();
+      b->bytes = n * bytes;
+      if (cudaMalloc(&b->p, b->bytes) == cudaSuccess) {
+        p = static_cast<double*>(b->p);
+        doubles = n * slice;
+        have = n;
+        bufs.push_back(std::move(b));
+        break;
+      }
+      b->p = nullptr;
+      cudaGetLastError();
+    }
+  }
+  return (int)std::min(want, have);
+}
+
 namespace {
 
 template <class T>
@@ -583,13 +609,6 @@ int ensure_buf(bg_op* op, double** p, size_t doubles) {
   return BG_OK;
 }
 
-// Units of a band density whose slices are formed before they are summed: all of them while
-// they fit in 1 GiB.
-int density_group(int units, int nk, const BoxGeo& g) {
-  const double slice = 8.0 * g.n0 * g.n1 * g.n2 * nk;
-  return (int)std::max(1.0, std::min((double)units, std::floor(1073741824.0 / slice)));
-}
-
 size_t grid_points(const bg_op* op) { return (size_t)op->dims[0] * op->dims[1] * op->dims[2]; }
 
 // Install a C-order grid (device pointer) into `dst` in the layout of t.vt; waits and
@@ -778,6 +797,13 @@ int bg_test_raise_error(bg_op* op, int32_t bits) {
   return e == cudaSuccess ? BG_OK : cuda_fail(op->ctx, e, "error word");
 }
 
+int bg_test_density_budget(bg_op* op, bg_kset* set, int64_t bytes) {
+  if (bytes < 0) return BG_EINVAL;
+  if (op) op->dens_part.budget = (size_t)bytes;
+  if (set) set->dens_part.budget = (size_t)bytes;
+  return BG_OK;
+}
+
 int bg_op_diagonal(const bg_op* op, double* out) {
   if (!op || !out) return fail(op ? op->ctx : nullptr, BG_EINVAL, "null argument");
   std::copy(op->diag.begin(), op->diag.end(), out);
@@ -947,9 +973,9 @@ int bg_op_band_density_sum(bg_op* op, const double* x, int64_t rows, int64_t col
     }
   } else {
     const int units = op->gamma ? (int)((cols + 1) / 2) : (int)cols;
-    const int group = density_group((int)op->cap_units, 1, op->g);  // the buffer's size, for any block
-    if ((rc = ensure_buf(op, &op->dens_part, (size_t)group * pts))) return rc;
-    if ((rc = ensure_buf(op, &op->dens_w, (size_t)op->cap))) return rc;
+    if ((rc = ensure_buf(op, &op->dens_w, (size_t)op->cap)) || (rc = ensure_buf(op, &op->dens_ksum, pts))) return rc;
+    const int group = op->dens_part.fit(pts, units, op->stream);
+    if (group == 0) return fail(ctx, BG_ENOMEM, "density slice");
     const size_t dpc = op->gamma ? (size_t)rows : (size_t)2 * rows;
     const double* dx = x;
     if (ptr_kind == BG_PTR_HOST) {
@@ -967,9 +993,8 @@ int bg_op_band_density_sum(bg_op* op, const double* x, int64_t rows, int64_t col
     a.ldx = a.ldy = (int64_t)dpc;
     a.cols = (int)cols;
     a.units = units;
-    if ((rc = ensure_buf(op, &op->dens_ksum, pts))) return rc;
     op->launches += launch_density(op->d_tabs, op->gamma ? 1 : 0, op->t.ngroups, op->g, bt, op->dens_w, 0, group, volume,
-                                   accumulate, op->dens_part, op->dens_ksum, dd, op->stream);
+                                   accumulate, op->dens_part.p, op->dens_ksum, dd, op->stream);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
   }
@@ -1118,7 +1143,6 @@ int bg_kset_destroy(bg_kset* ks) {
   cudaFree(ks->d_errs);
   cudaFree(ks->d_errv);
   if (ks->h_errv) cudaFreeHost(ks->h_errv);
-  cudaFree(ks->dens_part);
   cudaFree(ks->dens_ksum);
   cudaFree(ks->dens_w);
   cudaFree(ks->d_tabs);
@@ -1208,7 +1232,6 @@ int bg_kset_band_density_sum(bg_kset* ks, const double* const* x, int64_t cols, 
     return BG_OK;
   }
   const int units = ks->gamma ? (int)((cols + 1) / 2) : (int)cols;
-  const int group = density_group(units, n, g);
   auto grow = [&](double** p, size_t* have, size_t need) -> int {
     if (*have >= need) return BG_OK;
     cudaFree(*p);
@@ -1222,9 +1245,10 @@ int bg_kset_band_density_sum(bg_kset* ks, const double* const* x, int64_t cols, 
     return BG_OK;
   };
   int rc;
-  if ((rc = grow(&ks->dens_part, &ks->dens_part_doubles, (size_t)n * group * pts))) return rc;
   if ((rc = grow(&ks->dens_w, &ks->dens_w_doubles, (size_t)n * cols))) return rc;
   if ((rc = grow(&ks->dens_ksum, &ks->dens_ksum_doubles, (size_t)n * pts))) return rc;
+  const int group = ks->dens_part.fit((size_t)n * pts, units, ks->stream);
+  if (group == 0) return fail(ctx, BG_ENOMEM, "density slice");
   e = cudaMemcpyAsync(ks->dens_w, weights, (size_t)n * cols * sizeof(double), cudaMemcpyHostToDevice, ks->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "copy in");
   Batch bt;
@@ -1240,7 +1264,7 @@ int bg_kset_band_density_sum(bg_kset* ks, const double* const* x, int64_t cols, 
     a.units = units;
   }
   ks->launches += launch_density(ks->d_tabs, ks->gamma, ks->max_groups, g, bt, ks->dens_w, (int)cols, group, volume,
-                                 accumulate, ks->dens_part, ks->dens_ksum, density, ks->stream);
+                                 accumulate, ks->dens_part.p, ks->dens_ksum, density, ks->stream);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
   return BG_OK;
 }

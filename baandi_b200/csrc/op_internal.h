@@ -28,6 +28,19 @@ struct DevBuf {
   }
 };
 
+// The slices of a band density's group of units (launch_density).  A buffer that has been
+// outgrown stays until its owner goes: captured launches may hold its address.
+struct DensitySlices {
+  double* p = nullptr;
+  size_t doubles = 0;
+  size_t budget = (size_t)1 << 30;  // bytes of a group
+  std::vector<std::unique_ptr<DevBuf>> bufs;
+  // The group for `units` units of `slice` doubles each, 0 without memory for one.  Grows the
+  // buffer (at least doubling it) to all units within the budget and a quarter of the free
+  // memory; under a stream capture, and where an allocation fails, the buffer serves as it is.
+  int fit(size_t slice, int units, cudaStream_t s);
+};
+
 struct bg_op {
   bg_ctx* ctx = nullptr;
   bool gamma = false;
@@ -61,7 +74,7 @@ struct bg_op {
   double* vchange = nullptr;
   double* grid = nullptr;
   double* dens_w = nullptr;
-  double* dens_part = nullptr;
+  DensitySlices dens_part;
   double* dens_ksum = nullptr;  // one grid: the reduction's per-k sum
   bool vtf_valid = false;  // t.vtf (the FP32 apply's potential) matches t.vt
   bg::TcNl tc;             // tensor-core nonlocal products (BG_PREC_TENSOR)
@@ -104,8 +117,7 @@ struct bg_kset {
   void (*dv_free)(void*) = nullptr;
   // bg_kset_set_potential_ptr / bg_kset_band_density_sum buffers (lazily allocated)
   double** d_vts = nullptr;     // every operator's t.vt
-  double* dens_part = nullptr;  // [k][chunk][grid]
-  size_t dens_part_doubles = 0;
+  DensitySlices dens_part;  // [k][unit of the group][grid]
   double* dens_ksum = nullptr;  // [k][grid]
   size_t dens_ksum_doubles = 0;
   double* dens_w = nullptr;     // [k][column]

@@ -25,6 +25,10 @@ int bg_test_residue_products(int32_t mode, int32_t count, const int64_t* shapes,
                              const int64_t* ldc, int32_t op, int32_t presplit, const int64_t* bounds,
                              int64_t wait_limit);
 
+/* Bytes of the slices that a band density of the operator or the set (either may be NULL) forms
+ * before it sums them; at least one unit's are formed. */
+int bg_test_density_budget(bg_op* op, bg_kset* set, int64_t bytes);
+
 /* Set bits of the operator's device error word, as a kernel that met the error would. */
 int bg_test_raise_error(bg_op* op, int32_t bits);
 

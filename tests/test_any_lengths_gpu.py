@@ -1,6 +1,6 @@
 """Apply and band density on boxes of every line length (csrc/fft_any.cuh, planes_any.cu) and of
 lengths outside it, against numpy's FFT: each length once along every axis, one and two plane
-blocks per SM, odd unit counts, chunks of several units.  Bound: FP64 transforms of up to 128^3
+blocks per SM, odd unit counts; densities in one group of units and in several.  Bound: FP64 transforms of up to 128^3
 points, errors of a few eps times log2 N of the column's norm (the suite's 1e-12 parity bound
 holds them with room; 1e-13 here)."""
 import numpy as np
@@ -48,9 +48,12 @@ def test_box(ctx, dims):
     assert np.linalg.norm(got - want) <= 1e-13 * np.linalg.norm(want)
     w = rng.uniform(0.1, 2.0, cols)
     rho_want = np.einsum("b,bxyz->xyz", w, np.abs(psi) ** 2) / 7.0
-    rho = op.band_density_sum(x, w, 7.0)           # chunks of several units
+    rho = op.band_density_sum(x, w, 7.0)
     assert np.linalg.norm(rho - rho_want) <= 1e-13 * np.linalg.norm(rho_want)
-    ks = KPointSet([op], ctx)                      # one unit per block
+    # groups of two units and a last one of one: the same sums in the same order
+    assert op._lib.bg_test_density_budget(op.handle, None, 2 * 8 * int(np.prod(dims))) == 0
+    assert np.array_equal(op.band_density_sum(x, w, 7.0), rho)
+    ks = KPointSet([op], ctx)
     ks.set_stream(torch.cuda.current_stream().cuda_stream)
     rho = ks.band_density_sum([torch.from_numpy(np.ascontiguousarray(x.T)).cuda()], w[None, :], 7.0)
     assert np.linalg.norm(rho.cpu().numpy() - rho_want) <= 1e-13 * np.linalg.norm(rho_want)
