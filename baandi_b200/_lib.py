@@ -138,6 +138,8 @@ SIGNATURES = {
     "bg_test_residue_product": [_i32, _i64, _i64, _i64, _p, _i64, _p, _i64, _p, _i64, _i32, _i32],
     "bg_test_residue_products": [_i32, _i32, _p, _p, _p, _p, _p, _p, _p, _i32, _i32, _p, _i64],
     "bg_test_raise_error": [_p, _i32],
+    "bg_test_memory": [_p, _i64, _i32],
+    "bg_test_residue_state": [_p, _p, _p, _p],
     "bg_test_density_budget": [_p, _p, _i64],
     "bg_zgemm_bf16x3": [_p, _i32, _i64, _i64, _i64, _p, _i64, _p, _i64, _p, _i64, _i32, _p],
     "bg_learned_set": [_p, _p],

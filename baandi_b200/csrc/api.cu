@@ -48,6 +48,16 @@ int report_error_bits(bg_ctx* ctx, int bits) {
 }
 }  // namespace bg
 
+bool bg::spare_memory(const bg_ctx* ctx, size_t bytes, bool solves) {
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const size_t reserve = total / 8 + (solves ? ctx->promised->load() : 0);
+  return std::min(free, ctx->test_free) >= reserve && std::min(free, ctx->test_free) - reserve >= bytes;
+}
+
 int DensitySlices::fit(size_t slice, int units, cudaStream_t s) {
   const size_t bytes = slice * sizeof(double), most = std::max<size_t>(1, budget / bytes);
   const size_t want = std::min<size_t>((size_t)units, most);
@@ -197,12 +207,13 @@ int ksplit_for(int64_t rows, int nproj, int64_t cols, int* kchunk) {
 }
 
 // The projector table as residue panels of the FP64 products (gemm_rns.cuh), constant for
-// the operator's lifetime.  Without memory for them the operator keeps the FP64 tiles.
+// the operator's lifetime.  Without spare memory for them the operator keeps the FP64 tiles.
 int residue_panels(bg_op* op, const double2* p, int nproj) {
   NlDev& N = op->nl;
   const int rows = (int)op->rows;
   const size_t bytes[4] = {rns::a_panel_bytes(nproj, rows), rns::a_panel_bytes(rows, nproj),
                            2 * sizeof(double) * (size_t)nproj, 2 * sizeof(double) * (size_t)rows};
+  if (!spare_memory(op->ctx, bytes[0] + bytes[1] + bytes[2] + bytes[3], true)) return BG_OK;
   std::unique_ptr<DevBuf> b[4];
   for (int i = 0; i < 4; ++i) {
     b[i] = std::make_unique<DevBuf>();
@@ -533,7 +544,6 @@ int build_op(bg_ctx* ctx, const bg_basis_desc* b, const bg_projectors* pr, int64
       if (ce == cudaSuccess)
         ce = tc::split_a(tc::kNN, pd, npw, (int)npw, nproj, const_cast<unsigned char*>(N.p_nn), nullptr);
       if (ce != cudaSuccess) return cuda_fail(ctx, ce, "projector panels");
-      if (rns::pays(nproj, capacity, npw, true) && (rc = residue_panels(op.get(), pd, nproj))) return rc;
     }
     N.p = d_dbl;
     op->shape.natoms = natoms;
@@ -574,6 +584,13 @@ int build_op(bg_ctx* ctx, const bg_basis_desc* b, const bg_projectors* pr, int64
     return fail(ctx, BG_ESHAPE, "FFT plane does not fit in shared memory");
   if ((rc = configure_kernels((size_t)dev_smem, (size_t)dev_smem)) != BG_OK)
     return fail(ctx, BG_EDEVICE, "cudaFuncSetAttribute failed");
+  // the six basis blocks of a solve of `capacity` bands (kset_davidson.cu), then what is optional
+  op->promised = 6 * es * (size_t)npw * 2 * (size_t)capacity;
+  op->promises = ctx->promised;
+  *op->promises += op->promised;
+  if (!gamma && op->shape.nproj > 0 && rns::pays(op->shape.nproj, capacity, npw, true) &&
+      (rc = residue_panels(op.get(), reinterpret_cast<const double2*>(op->nl.p), op->shape.nproj)))
+    return rc;
   if ((rc = upload(op.get(), &op->t, 1, &op->d_tabs))) return rc;
   if ((rc = upload(op.get(), &op->nl, 1, &op->d_nl))) return rc;
   for (int i = 0; i < 2 * kStages; ++i)
@@ -763,7 +780,7 @@ int bg_op_apply_block(bg_op* op, const double* x, double* y, int64_t rows, int64
   if (tensor_nl) {
     op->launches += launch_nonlocal_tc(op->d_nl, op->shape, (int)op->rows, (int)cols, bt, &op->tc, op->stream, &op->ev);
   } else if (op->shape.nproj > 0 && op->nl.r_tn && rns::pays(op->shape.nproj, cols, op->rows, true) &&
-             ensure_nonlocal_rns(&op->rns, 1, op->shape.nproj, op->cap, (int)op->rows, op->stream)) {
+             ensure_nonlocal_rns(&op->rns, 1, op->shape.nproj, op->cap, (int)op->rows, op->stream, ctx, true)) {
     op->launches += launch_nonlocal_rns(op->d_nl, op->shape, (int)op->rows, (int)cols, bt, &op->rns, op->t.err,
                                         op->stream, &op->ev);
   } else if (op->shape.nproj > 0) {
@@ -795,6 +812,19 @@ int bg_test_raise_error(bg_op* op, int32_t bits) {
   word |= bits;
   if (e == cudaSuccess) e = cudaMemcpy(op->t.err, &word, sizeof(int), cudaMemcpyHostToDevice);
   return e == cudaSuccess ? BG_OK : cuda_fail(op->ctx, e, "error word");
+}
+
+int bg_test_memory(bg_ctx* ctx, int64_t free_bytes, int32_t failures) {
+  if (!ctx) return BG_EINVAL;
+  ctx->test_free = free_bytes < 0 ? SIZE_MAX : (size_t)free_bytes;
+  ctx->test_failures = failures;
+  return BG_OK;
+}
+
+int bg_test_residue_state(const bg_op* op, const bg_kset* set, int32_t* panels, int32_t* products) {
+  if (panels) *panels = op && op->nl.r_tn ? 1 : 0;
+  if (products) *products = set && set->dv_residues ? 1 : 0;
+  return BG_OK;
 }
 
 int bg_test_density_budget(bg_op* op, bg_kset* set, int64_t bytes) {
@@ -1029,7 +1059,7 @@ static bool residue_products(bg_kset* ks, int k0, int k1, int64_t max_cols, int 
     if (!ks->ops[k]->nl.r_tn) return false;
   int64_t cap = 0;
   for (const bg_op* o : ks->ops) cap = std::max(cap, o->cap);
-  return ensure_nonlocal_rns(r, (int)ks->ops.size(), ks->shape.nproj, cap, ks->max_rows, s);
+  return ensure_nonlocal_rns(r, (int)ks->ops.size(), ks->shape.nproj, cap, ks->max_rows, s, ks->ctx, true);
 }
 
 int enqueue_range(bg_kset* ks, int k0, int k1, const CallArgs* args, const int64_t* cols, cudaStream_t s,

@@ -7,6 +7,8 @@
 
 #include "fft_dev.cuh"
 
+struct bg_ctx;
+
 namespace bg {
 
 // Immutable per-operator tables, resident in HBM.  The FFT box is n0 x n1 x n2
@@ -175,10 +177,15 @@ struct RnsNl {
   bool tried = false;
   void release();
 };
+// Whether `bytes` of device memory may go to buffers that only make calls faster: an eighth of
+// the device stays free, and (`solves`) the work arrays of one solve over every operator of the
+// context, so that what the calls need still fits.
+bool spare_memory(const bg_ctx* ctx, size_t bytes, bool solves);
 // True when the buffers are ready for blocks of up to max_cols columns (the same bound on
-// every call).  Allocates on the first call outside a stream capture; a failed allocation
-// leaves the FP64 tiles in use.
-bool ensure_nonlocal_rns(RnsNl* r, int nk, int nproj, int64_t max_cols, int max_rows, cudaStream_t s);
+// every call).  Allocates on the first call outside a stream capture; without spare memory
+// (solves: as spare_memory) the FP64 tiles stay in use.
+bool ensure_nonlocal_rns(RnsNl* r, int nk, int nproj, int64_t max_cols, int max_rows, cudaStream_t s,
+                         const bg_ctx* ctx, bool solves);
 // Enqueue y += P (D (P^H x)) with both products as residue products (complex operators
 // with panels); err: the device error word of a wait that gave up.
 int launch_nonlocal_rns(const NlDev* nl, const NlShape& sh, int max_rows, int max_cols, const Batch& b, RnsNl* r,

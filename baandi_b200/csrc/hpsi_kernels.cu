@@ -1094,7 +1094,8 @@ void RnsNl::release() {
   desc = work = nullptr;
 }
 
-bool ensure_nonlocal_rns(RnsNl* r, int nk, int nproj, int64_t max_cols, int max_rows, cudaStream_t s) {
+bool ensure_nonlocal_rns(RnsNl* r, int nk, int nproj, int64_t max_cols, int max_rows, cudaStream_t s,
+                         const bg_ctx* ctx, bool solves) {
   if (r->work) return true;
   if (r->tried) return false;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
@@ -1107,6 +1108,7 @@ bool ensure_nonlocal_rns(RnsNl* r, int nk, int nproj, int64_t max_cols, int max_
   // the workspace
   const size_t need = std::max(rns::workspace_bytes(rns::kTN, nk, nproj, (int)max_cols, max_rows, true),
                                rns::workspace_bytes(rns::kNN, nk, max_rows, (int)max_cols, nproj, true));
+  if (!spare_memory(ctx, need, solves)) return false;
   if (rns::prepare() != cudaSuccess || cudaMalloc(&r->desc, sizeof(rns::Desc) * 2 * kMaxBatch) != cudaSuccess ||
       cudaMalloc(&r->work, need) != cudaSuccess) {
     cudaGetLastError();

@@ -1426,6 +1426,7 @@ class KsetSolver {
     o_.cap = cap;
     o_.smem_matrices = small(cap) ? 1 : 0;
     o_.wide = wide ? 1 : 0;
+    ks_->dv_residues = false;
   }
   bool matches(int n, int cap, bool wide) const { return o_.n == n && o_.cap == cap && wide_ == wide; }
   // Per-call options (threshold, occupied, first_step, iterations, preconditioner).
@@ -1482,6 +1483,7 @@ class KsetSolver {
   Opts o_;
   bool want_graph_ = true;
   bool prepared_ = false;
+  bool residues_tried_ = false;
   bool graph_tried_[3] = {false, false, false};   // by precision (0 FP64, 1 FP32, 2 tensor)
   Opts* d_opts_ = nullptr;
   cudaStream_t s_ = nullptr;
@@ -1513,7 +1515,9 @@ class KsetSolver {
   template <class P>
   int alloc(P** p, size_t count) {
     void* q = nullptr;
-    if (cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(P)) != cudaSuccess) {
+    if ((ks_->ctx->test_failures > 0 && ks_->ctx->test_failures--) ||
+        cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(P)) != cudaSuccess) {
+      cudaGetLastError();
       err_ = "cudaMalloc failed";
       return BG_ENOMEM;
     }
@@ -1575,10 +1579,12 @@ class KsetSolver {
     return l + 1 + tc::launch_zgemm(tc::kTN, d_tctn_, nslots * nk_, o_.cap, o_.cap, max_rows_, tc_ks_, false, tc_work_,
                                 tc_err_, s_);
   }
-  // Buffers of the residue products (once, before any capture), where the largest Gram or
-  // rotation pays; without memory for them every product stays on the FP64 tiles.
+  // Buffers of the residue products (once, before any capture, after everything a solve
+  // cannot do without), where the largest Gram or rotation pays; without spare memory for
+  // them every product stays on the FP64 tiles.
   void prepare_residues() {
-    if (sizeof(D) != sizeof(double2)) return;
+    if (residues_tried_ || sizeof(D) != sizeof(double2)) return;
+    residues_tried_ = true;
     if (!ks_->dense && ks_->shape.nproj > 0 && rns::pays(ks_->shape.nproj, o_.n, max_rows_, true)) {
       bool panels = true;
       int64_t cap = 0;
@@ -1586,13 +1592,14 @@ class KsetSolver {
         panels = panels && op->nl.r_tn;
         cap = std::max(cap, op->cap);
       }
-      if (panels) ensure_nonlocal_rns(&rnsnl_, nk_, ks_->shape.nproj, o_.n, max_rows_, s_);
+      if (panels) ensure_nonlocal_rns(&rnsnl_, nk_, ks_->shape.nproj, o_.n, max_rows_, s_, ks_->ctx, false);
     }
     if (2 * nk_ > 128 || !rns::pays(o_.cap, o_.n, max_rows_, false)) return;
     static_assert(kNnSlots == 2 && kTnSlots == 2, "descriptor slots");
     const size_t need = std::max(rns::workspace_bytes(rns::kTN, 2 * nk_, o_.cap, o_.n, max_rows_, false),
                                  rns::workspace_bytes(rns::kNN, 2 * nk_, max_rows_, o_.n, o_.cap, false));
     void *d = nullptr, *w = nullptr;
+    if (!spare_memory(ks_->ctx, need, false)) return;
     if (rns::prepare() != cudaSuccess || cudaMalloc(&d, sizeof(rns::Desc) * 2 * nk_) != cudaSuccess ||
         cudaMalloc(&w, need) != cudaSuccess) {
       cudaGetLastError();
@@ -1604,6 +1611,28 @@ class KsetSolver {
     d_rns_ = static_cast<rns::Desc*>(d);
     rns_work_ = static_cast<unsigned char*>(w);
     rns_bytes_ = need;
+    ks_->dv_residues = true;
+  }
+  // Gives the residue products' buffers back (the captured iterations with them, which hold
+  // their addresses) when something a solve cannot do without has found no memory.
+  void drop_residues() {
+    cudaStreamSynchronize(s_);
+    for (int p = 0; p < 3; ++p) {
+      if (exec_[p]) cudaGraphExecDestroy(exec_[p]);
+      if (graph_[p]) cudaGraphDestroy(graph_[p]);
+      exec_[p] = nullptr;
+      graph_[p] = nullptr;
+      graph_tried_[p] = false;
+    }
+    for (void* p : {(void*)d_rns_, (void*)rns_work_}) {
+      dev_.erase(std::remove(dev_.begin(), dev_.end(), p), dev_.end());
+      cudaFree(p);
+    }
+    d_rns_ = nullptr;
+    rns_work_ = nullptr;
+    rnsnl_.release();
+    rnsnl_.tried = true;
+    ks_->dv_residues = false;
   }
   // Buffers of the precision form (once, before any capture).
   int prepare_tensor() {
@@ -1805,7 +1834,6 @@ int KsetSolver<T>::prepare() {
   }
   if ((rc = cuda(cudaMemcpy(d_bufs_, hb_.data(), sizeof(Bufs<D>) * nk_, cudaMemcpyHostToDevice), "upload")))
     return rc;
-  prepare_residues();
   args_.assign(nk_, CallArgs{});
   cols_.assign(nk_, n);
   for (int k = 0; k < nk_; ++k) {
@@ -1833,7 +1861,13 @@ int KsetSolver<T>::solve(const double* const* start, const double* const* diagon
   s_ = ks_->stream;
   launches_ = 0;
   if (!prepared_ && (rc = prepare())) return rc;
-  if (o_.tensor && (rc = prepare_tensor())) return rc;
+  if (o_.tensor && (rc = prepare_tensor())) {
+    if (rc != BG_ENOMEM || (!rns_work_ && !rnsnl_.work)) return rc;
+    drop_residues();
+    if ((rc = prepare_tensor())) return rc;
+    err_.clear();
+  }
+  prepare_residues();
   // the pinned pointer table may still feed a copy of the previous solve
   if ((rc = cuda(cudaStreamSynchronize(s_), "start"))) return rc;
   for (int k = 0; k < nk_; ++k) {

@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
+#include <cstdint>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -15,6 +17,11 @@ struct bg_ctx {
   std::string error;
   std::mutex mu;
   void* learned = nullptr;  // BF16 parameters of the learned preconditioner (device), or null
+  // bytes of the work arrays of one solve over every operator alive (spare_memory)
+  std::shared_ptr<std::atomic<size_t>> promised = std::make_shared<std::atomic<size_t>>(0);
+  // tests: what spare_memory takes for free at most, and how many allocations of a solver fail
+  size_t test_free = SIZE_MAX;
+  int test_failures = 0;
   ~bg_ctx() {
     if (learned) cudaFree(learned);
   }
@@ -53,6 +60,11 @@ struct bg_op {
   int64_t launches = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  size_t promised = 0;  // this operator's part of the context's count
+  std::shared_ptr<std::atomic<size_t>> promises;
+  ~bg_op() {
+    if (promises) *promises -= promised;
+  }
   std::vector<double> diag;
   bg::OpTables t{};
   bg::BoxGeo g{};
@@ -128,6 +140,7 @@ struct bg_kset {
   int* h_errv = nullptr;
   bg::TcNl tc;  // tensor-core nonlocal products (BG_PREC_TENSOR)
   bg::RnsNl rns;  // FP64 nonlocal products on the int8 tensor cores
+  bool dv_residues = false;  // the cached solver's Grams and rotations have residue buffers
 };
 
 namespace bg {

@@ -93,7 +93,12 @@ typedef struct {
 } bg_projectors;
 
 /* Replaces DistributedComplexHamiltonian::new_owned (distributed_complex.rs:88-167)
- * with one rank.  capacity = widest block bg_op_apply_block accepts. */
+ * with one rank.  capacity = widest block bg_op_apply_block accepts.
+ * Device memory beyond the tables: FP64 products of large complex operators run faster from
+ * residue panels of the projector table (64 bytes per complex element, 4.6 GB for 864
+ * projectors x 80,725 plane waves, made here) and from workspaces of the first apply and solve.
+ * They are taken only while an eighth of the device's memory, and the work arrays of one solve
+ * over every operator of the context, stay free; otherwise the calls run without them. */
 int bg_op_create_complex(bg_ctx* ctx, const bg_basis_desc* basis, const bg_projectors* proj,
                          int64_t capacity, bg_op** out);
 

@@ -29,6 +29,15 @@ int bg_test_residue_products(int32_t mode, int32_t count, const int64_t* shapes,
  * before it sums them; at least one unit's are formed. */
 int bg_test_density_budget(bg_op* op, bg_kset* set, int64_t bytes);
 
+/* Short memory: what the library takes for free device memory at most when it decides on buffers
+ * that only make calls faster (negative: what the device says), and how many of the next
+ * allocations of a batched Davidson solver fail. */
+int bg_test_memory(bg_ctx* ctx, int64_t free_bytes, int32_t failures);
+
+/* Whether the operator holds residue panels of its projectors, and whether the set's last solve
+ * formed its large products as residue products (either output may be NULL). */
+int bg_test_residue_state(const bg_op* op, const bg_kset* set, int32_t* panels, int32_t* products);
+
 /* Set bits of the operator's device error word, as a kernel that met the error would. */
 int bg_test_raise_error(bg_op* op, int32_t bits);
 
