@@ -817,28 +817,25 @@ __global__ void __launch_bounds__(kT) k_w_tri_gs(const Bufs<D>* __restrict__ buf
   }
 }
 
-// Y[:, c] = H_0 H_1 ... H_{m-3} (s . Z[:, order[c]]) for c < m: kBackCols columns per
-// block, one warp per column; each reflector is staged once per block in shared memory
+// Y[:, c] = H_0 H_1 ... H_{m-3} (s . Z[:, order[c]]) for c < m: `cols` columns per block, one warp per column; each reflector is staged once per block in shared memory
 // (double-buffered, one barrier per reflector) and applied by every warp to its column.
-// 7: the 960 columns of the Si216 problem are 138 blocks, one wave of the 148 SMs (a block takes
-// most of an SM's shared memory); 6 columns made 160 blocks run two waves, 2.0 ms a call.
-constexpr int kBackCols = 7;  // (7 + 2) x 1152 x 16 bytes of shared memory at the largest capacity
 template <class D>
-__global__ void __launch_bounds__(kT) k_w_back(const Bufs<D>* __restrict__ bufs, const Ctl* __restrict__ ctl, int cap) {
+__global__ void __launch_bounds__(kT) k_w_back(const Bufs<D>* __restrict__ bufs, const Ctl* __restrict__ ctl, int cap,
+                                               int cols) {
   using X = Cx<D>;
   const int k = blockIdx.y;
   const Ctl c = ctl[k];
   const Bufs<D> b = bufs[k];
   if (c.status != 0 || c.we_m == 0 || *(volatile int*)b.werr != 0) return;
   const int m = c.we_m;
-  const int c0 = blockIdx.x * kBackCols;
+  const int c0 = blockIdx.x * cols;
   if (c0 >= m) return;
   extern __shared__ __align__(16) unsigned char w_sm[];
-  D* z = reinterpret_cast<D*>(w_sm);          // [kBackCols][cap]
-  D* vb = z + (size_t)kBackCols * cap;        // two reflector buffers of cap
+  D* z = reinterpret_cast<D*>(w_sm);          // [cols][cap]
+  D* vb = z + (size_t)cols * cap;        // two reflector buffers of cap
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = c0 + warp;
-  const bool act = warp < kBackCols && col < m;
+  const bool act = warp < cols && col < m;
   D* zc = z + (size_t)warp * cap;
   if (act) {
     const int src = b.order[col];
@@ -867,7 +864,30 @@ __global__ void __launch_bounds__(kT) k_w_back(const Bufs<D>* __restrict__ bufs,
     for (int r = lane; r < m; r += 32) b.Y[r + (size_t)col * cap] = zc[r];
 }
 
-inline size_t back_smem(int cap, size_t dsize) { return ((size_t)kBackCols + 2) * cap * dsize; }
+inline size_t back_smem(int cols, int cap, size_t dsize) { return ((size_t)cols + 2) * cap * dsize; }
+// Columns per block of k_w_back: the fewest whose blocks run in the fewest waves.  A block's time
+// hardly depends on its columns (each has a warp), a second wave doubles it: the complex reduced
+// problem of m = 960 takes 17.8 ms with 4 or 7 columns (one wave) and 19.7 with 2 or 6 (two),
+// m = 1152 23.3 with 4 or 8 and 26.2 with 1 to 3 or 5 to 7; up to m = 640 any count gives one wave
+// and times within 1 %.
+template <class D>
+int back_cols(int cap, int nk, int sms) {
+  int best = 1;
+  int64_t fewest = INT64_MAX;
+  for (int cols = 1; cols <= kT / 32; ++cols) {
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_w_back<D>, kT, back_smem(cols, cap, sizeof(D))) !=
+            cudaSuccess || occ < 1)
+      break;
+    const int64_t slots = (int64_t)sms * occ, blocks = (int64_t)((cap + cols - 1) / cols) * nk;
+    const int64_t waves = (blocks + slots - 1) / slots;
+    if (waves < fewest) {
+      fewest = waves;
+      best = cols;
+    }
+  }
+  return best;
+}
 
 // LT = L^H (m x m).
 template <class D>
@@ -901,7 +921,7 @@ int prepare(int cap, int* coop_blocks, std::string* err) {
                              (int)house_smem(cap, std::max(sms0, 1), sizeof(D)));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute((const void*)k_w_back<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)back_smem(cap, sizeof(D)));
+                             (int)back_smem(kT / 32, cap, sizeof(D)));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute((const void*)k_w_trsm<D, kSolveBorder>, cudaFuncAttributeMaxDynamicSharedMemorySize, tsm);
   if (e == cudaSuccess)
@@ -962,8 +982,9 @@ int64_t launch_eig(Bufs<D>* bufs, Ctl* ctl, int nk, int cap, int coop_blocks, un
   k_w_tri_clusters<D><<<dim3(1, (unsigned)nk), 256, 0, s>>>(bufs, ctl);
   k_w_tri_vectors<D><<<dim3((unsigned)((cap + 63) / 64), (unsigned)nk), 64, 0, s>>>(bufs, ctl, cap);
   k_w_tri_gs<D><<<gw, kT, 0, s>>>(bufs, ctl, cap);
-  k_w_back<D><<<dim3((unsigned)((cap + kBackCols - 1) / kBackCols), (unsigned)nk), kT, back_smem(cap, sizeof(D)), s>>>(
-      bufs, ctl, cap);
+  const int cols = back_cols<D>(cap, nk, coop_blocks);
+  k_w_back<D><<<dim3((unsigned)((cap + cols - 1) / cols), (unsigned)nk), kT, back_smem(cols, cap, sizeof(D)), s>>>(
+      bufs, ctl, cap, cols);
   k_w_adjoint<D><<<dim3(256, (unsigned)nk), 256, 0, s>>>(bufs, ctl, cap);
   k_w_trsm<D, kSolveBack><<<gs, kT, tsm, s>>>(bufs, ctl, cap);
   return 12;

@@ -56,6 +56,18 @@ def test_reduced_eigh_matches_numpy(ctx, m, complex_):
     assert ms > 0.0
 
 
+@pytest.mark.parametrize("m,complex_", [(1, True), (3, False), (149, False), (301, True), (741, True), (1152, False)])
+def test_reduced_eigh_column_blocks(ctx, m, complex_):
+    """The back-transformation's columns per block follow from the size (back_cols): sizes on both
+    sides of a wave, ragged last blocks, the smallest and the largest, by residual and Gram."""
+    h, s = _clustered_pencil(m, complex_, 3 + m)
+    w, c, _ = DV.reduced_eigh(s, h, ctx)
+    scale = max(1.0, np.max(np.abs(w)))
+    assert np.max(np.abs(c.conj().T @ s @ c - np.eye(m))) <= 1e-10
+    assert np.max(np.abs(h @ c - (s @ c) * w[None, :])) <= 1e-10 * scale
+    assert np.all(np.diff(w) >= 0.0)
+
+
 def test_reduced_eigh_rejects_dependent_overlap(ctx):
     from baandi_b200.hamiltonian import SolverError
     m = 64
