@@ -2,6 +2,7 @@
 //
 // Passes of one launch:
 //   k_rns_scale_cols / _rows  power-of-two scale of every operand column or row (2-norm)
+//   k_rns_balance             power-of-two balance of K (A B products that split A)
 //   k_rns_split               integers, modulo the moduli, as int8 panels in MMA tile order
 //   k_rns_mma                 the 2 kModuli int8 products; epilogue reduces to one byte
 //   k_rns_join                Chinese remainder: bytes -> FP64, C (op)= result
@@ -104,7 +105,7 @@ constexpr Tables make_tables() {
   return t;
 }
 constexpr Tables kTab = make_tables();
-static_assert(kTab.mhi > 2.6e35 && 2.0 * kNormBits + 1.0 < kLog2M, "2^117.69 < product of the moduli");
+static_assert(kTab.mhi > 2.6806e35 && 2.0 * kNormBits + 1.0 < kLog2M, "2^117.69 = 2.6805e35 < product of the moduli");
 __constant__ Tables c_tab = make_tables();
 
 // --------------------------------------------------------------------- PTX
@@ -205,10 +206,20 @@ __device__ __forceinline__ void scale_of(double ssq, double amax, double n, doub
   *inv = ldexp(1.0, -(int)e);
 }
 
-struct Operand {  // element (row j, K index k) at X[k sk + j sj]
+struct Operand {  // element (row j, K index k): X[k sk + j sj] bal[k]
   const double2* X;
   int64_t sk, sj;
   int rows, K;
+  const double* bal = nullptr;  // (BAL)
+  template <bool BAL>
+  __device__ __forceinline__ double2 balanced(double2 v, int k) const {
+    if constexpr (BAL) {
+      const double s = __ldg(bal + k);
+      v.x *= s;
+      v.y *= s;
+    }
+    return v;
+  }
 };
 __device__ __forceinline__ Operand operand_of(const Desc& d, int mode, int which) {
   Operand o;
@@ -228,13 +239,14 @@ __device__ __forceinline__ Operand operand_of(const Desc& d, int mode, int which
 }
 
 // One block per row whose K run is contiguous (columns of A and B).
+template <bool BAL>
 __device__ __forceinline__ void scale_cols(const Operand& o, int j, double* sc, double* inv) {
   __shared__ double s_sum[8], s_max[8];
   const double2* x = o.X + (int64_t)j * o.sj;
   double ssq = 0.0, amax = 0.0;
 #pragma unroll 4
   for (int k = threadIdx.x; k < o.K; k += 256) {
-    const double2 v = __ldg(x + k);
+    const double2 v = o.template balanced<BAL>(__ldg(x + k), k);
     ssq = fma(v.x, v.x, fma(v.y, v.y, ssq));
     amax = fmax(amax, fmax(fabs(v.x), fabs(v.y)));
   }
@@ -255,7 +267,32 @@ __device__ __forceinline__ void scale_cols(const Operand& o, int j, double* sc, 
     scale_of(ssq, amax, o.K, sc + j, inv + j);
   }
 }
+// d[k] = the largest of |B_kj| over the columns j, each relative to its column's norm (the power
+// of two below it); dinv = 1 / d.  A D and D^-1 B have the product A B, but a row of A D counts
+// its entries as the product does: coefficients of 1e-8 on large entries no longer set the
+// quantum of the row's others.  32 K indices x 8 column slices per block.
+__device__ __forceinline__ void balance(const Operand& o, const double* sc, double* d, double* dinv) {
+  __shared__ double b_max[8][32];
+  const int kl = threadIdx.x & 31, q = threadIdx.x >> 5, k = blockIdx.x * 32 + kl;
+  double m = 0.0;
+  if (k < o.K) {
+#pragma unroll 8
+    for (int j = q; j < o.rows; j += 8) {
+      const double2 v = __ldg(o.X + k + (int64_t)j * o.sj);
+      m = fmax(m, fmax(fabs(v.x), fabs(v.y)) * sc[j]);  // a row with a NaN or an infinity has scale 0: skipped
+    }
+  }
+  b_max[q][kl] = m;
+  __syncthreads();
+  if (q == 0 && k < o.K) {
+    for (int w = 1; w < 8; ++w) m = fmax(m, b_max[w][kl]);
+    const int e = m >= 1.0 ? min(0, ilogb(m) - (int)kNormBits) : -(int)kNormBits;
+    d[k] = ldexp(1.0, e);
+    dinv[k] = ldexp(1.0, -e);
+  }
+}
 // 64 rows x 4 K quarters per block, rows contiguous in memory (rows of A in A B).
+template <bool BAL>
 __device__ __forceinline__ void scale_rows(const Operand& o, int j0, double* sc, double* inv) {
   __shared__ double r_sum[4][64], r_max[4][64];
   const int jl = threadIdx.x & 63, q = threadIdx.x >> 6, j = j0 + jl;
@@ -264,7 +301,7 @@ __device__ __forceinline__ void scale_rows(const Operand& o, int j0, double* sc,
     const double2* x = o.X + j;
 #pragma unroll 8
     for (int k = q; k < o.K; k += 4) {
-      const double2 v = __ldg(x + (int64_t)k * o.sk);
+      const double2 v = o.template balanced<BAL>(__ldg(x + (int64_t)k * o.sk), k);
       ssq = fma(v.x, v.x, fma(v.y, v.y, ssq));
       amax = fmax(amax, fmax(fabs(v.x), fabs(v.y)));
     }
@@ -286,11 +323,12 @@ __device__ __forceinline__ void scale_rows(const Operand& o, int j0, double* sc,
 // 16-byte chunk): integers v = rint(x scale) with |v| < 2^59, their eight bytes (of
 // v + 2^63) against the powers of 256 modulo p by dp4a (real part w, imaginary part r w),
 // z+- = a +- r b, one rounded multiple of p taken off through a float, and one 8-byte store
-// per plane.  Bound by these ~14 integer and float operations per value and modulus, close
-// to the panels' store bandwidth.
+// per plane.  Bound by these ~14 integer and float operations per value and modulus (0.59 of the
+// copy rate; 64 registers with a small spill, for two 512-thread blocks per SM).
 __device__ __forceinline__ unsigned pack4(const unsigned* b) {  // low bytes of four words
   return __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
 }
+template <bool BAL>
 __device__ __forceinline__ void split_rows(const Operand& o, bool conj, int R, int rt, int rt_n, int ktc,
                                            const double* __restrict__ scale, unsigned char* panel) {
   const int r = threadIdx.x >> 1, h = threadIdx.x & 1;
@@ -305,7 +343,7 @@ __device__ __forceinline__ void split_rows(const Operand& o, bool conj, int R, i
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       x[u] = make_double2(0.0, 0.0);
-      if (j < o.rows && k0 + u < o.K) x[u] = __ldg(o.X + (int64_t)(k0 + u) * o.sk + (int64_t)j * o.sj);
+      if (j < o.rows && k0 + u < o.K) x[u] = o.template balanced<BAL>(__ldg(o.X + (int64_t)(k0 + u) * o.sk + (int64_t)j * o.sj), k0 + u);
     }
     unsigned al[8], ah[8], bl[8], bh[8];
 #pragma unroll
@@ -351,50 +389,69 @@ struct Geo {
   int max_m, max_n;
   size_t a_stride, b_stride, r_stride;  // bytes per descriptor (residues: all splits)
   size_t a_off, b_off, r_off, as_off, bs_off, total;  // byte offsets in the workspace
+  int max_k;        // balance of K (kNN, A split with the launch): d and 1 / d per K index
+  size_t bal_off;   // 0: none
 };
+__device__ __forceinline__ double* balance_of(const Geo& g, unsigned char* work, int z) {
+  return reinterpret_cast<double*>(work + g.bal_off) + 2 * (size_t)z * g.max_k;
+}
 
+// BAL: with the balance of K (the second pass over B)
+template <bool BAL>
 __global__ void __launch_bounds__(256) k_rns_scale_cols(const Desc* __restrict__ descs, int mode, int which, Geo g,
                                                         unsigned char* work) {
   const Desc d = descs[blockIdx.y];
   if (d.M <= 0 || d.N <= 0 || d.K <= 0 || (which == 0 && d.a_panel)) return;
-  const Operand o = operand_of(d, mode, which);
+  Operand o = operand_of(d, mode, which);
   if ((int)blockIdx.x >= o.rows) return;
+  if (BAL) o.bal = balance_of(g, work, blockIdx.y) + g.max_k;
   const int cap = which == 0 ? g.max_m : g.max_n;
   double* sc = reinterpret_cast<double*>(work + (which == 0 ? g.as_off : g.bs_off)) + 2 * (size_t)blockIdx.y * cap;
-  scale_cols(o, blockIdx.x, sc, sc + cap);
+  scale_cols<BAL>(o, blockIdx.x, sc, sc + cap);
 }
 __global__ void __launch_bounds__(256) k_rns_scale_rows(const Desc* __restrict__ descs, int mode, Geo g,
                                                         unsigned char* work) {
   const Desc d = descs[blockIdx.y];
   if (d.M <= 0 || d.N <= 0 || d.K <= 0 || d.a_panel) return;
-  const Operand o = operand_of(d, mode, 0);
+  Operand o = operand_of(d, mode, 0);
   if ((int)blockIdx.x * 64 >= o.rows) return;
+  o.bal = balance_of(g, work, blockIdx.y);
   double* sc = reinterpret_cast<double*>(work + g.as_off) + 2 * (size_t)blockIdx.y * g.max_m;
-  scale_rows(o, blockIdx.x * 64, sc, sc + g.max_m);
+  scale_rows<true>(o, blockIdx.x * 64, sc, sc + g.max_m);
+}
+__global__ void __launch_bounds__(256) k_rns_balance(const Desc* __restrict__ descs, int mode, Geo g,
+                                                     unsigned char* work) {
+  const Desc d = descs[blockIdx.y];
+  if (d.M <= 0 || d.N <= 0 || d.K <= 0 || (int)blockIdx.x * 32 >= d.K) return;
+  const double* sc = reinterpret_cast<const double*>(work + g.bs_off) + 2 * (size_t)blockIdx.y * g.max_n;
+  double* bal = balance_of(g, work, blockIdx.y);
+  balance(operand_of(d, mode, 1), sc, bal, bal + g.max_k);
 }
 __global__ void __launch_bounds__(256) k_rns_scale_args(Operand o, int by_rows, double* sc, double* inv) {
   if (by_rows)
-    scale_rows(o, blockIdx.x * 64, sc, inv);
+    scale_rows<false>(o, blockIdx.x * 64, sc, inv);
   else
-    scale_cols(o, blockIdx.x, sc, inv);
+    scale_cols<false>(o, blockIdx.x, sc, inv);
 }
 
+template <bool BAL>
 __global__ void __launch_bounds__(512, 2) k_rns_split(const Desc* __restrict__ descs, int mode, int which, Geo g,
                                                       unsigned char* work) {
   const Desc d = descs[blockIdx.z];
   if (d.M <= 0 || d.N <= 0 || d.K <= 0 || (which == 0 && d.a_panel)) return;
-  const Operand o = operand_of(d, mode, which);
+  Operand o = operand_of(d, mode, which);
+  if (BAL) o.bal = balance_of(g, work, blockIdx.z) + (which == 0 ? 0 : g.max_k);
   const int R = which == 0 ? kTileM : g.trb, rt_n = which == 0 ? g.a_mt : g.nt;
   if ((int)blockIdx.y * R >= o.rows) return;
   const int cap = which == 0 ? g.max_m : g.max_n;
   const double* sc =
       reinterpret_cast<const double*>(work + (which == 0 ? g.as_off : g.bs_off)) + 2 * (size_t)blockIdx.z * cap;
   unsigned char* panel = work + (which == 0 ? g.a_off + blockIdx.z * g.a_stride : g.b_off + blockIdx.z * g.b_stride);
-  split_rows(o, which == 0 && mode == kTN, R, blockIdx.y, rt_n, g.ktc, sc, panel);
+  split_rows<BAL>(o, which == 0 && mode == kTN, R, blockIdx.y, rt_n, g.ktc, sc, panel);
 }
 __global__ void __launch_bounds__(512, 2) k_rns_split_args(Operand o, int conj, int rt_n, int ktc,
                                                            const double* __restrict__ sc, unsigned char* panel) {
-  split_rows(o, conj != 0, kTileM, blockIdx.y, rt_n, ktc, sc, panel);
+  split_rows<false>(o, conj != 0, kTileM, blockIdx.y, rt_n, ktc, sc, panel);
 }
 
 // --------------------------------------------------------------------- product
@@ -809,6 +866,11 @@ Geo carve(int mode, int ndesc, int max_m, int max_n, int max_k, bool a_presplit,
   o += round256(a_presplit ? 0 : (size_t)ndesc * 2 * max_m * sizeof(double));
   g.bs_off = o;
   o += round256((size_t)ndesc * 2 * max_n * sizeof(double));
+  g.max_k = max_k;
+  if (mode == kNN && !a_presplit) {
+    g.bal_off = o;
+    o += round256((size_t)ndesc * 2 * max_k * sizeof(double));
+  }
   g.r_off = o;
   const int least = (max_k + kMaxK - 1) / kMaxK;
   for (g.ksplit = pick_ksplit(mode, ndesc, max_m, max_n, max_k, g.trb);; --g.ksplit) {
@@ -842,19 +904,33 @@ int launch_product(int mode, const Desc* d_desc, int ndesc, int max_m, int max_n
   unsigned char* w = static_cast<unsigned char*>(work);
   int launches = 4;
   const unsigned chunks = (unsigned)(4 * g.ktc);
+  auto split = [&](unsigned gx, int tiles, int threads, int which) {
+    if (g.bal_off)
+      k_rns_split<true><<<dim3(gx, tiles, ndesc), threads, 0, s>>>(d_desc, mode, which, g, w);
+    else
+      k_rns_split<false><<<dim3(gx, tiles, ndesc), threads, 0, s>>>(d_desc, mode, which, g, w);
+  };
+  if (g.bal_off) {
+    k_rns_scale_cols<false><<<dim3(max_n, ndesc), 256, 0, s>>>(d_desc, mode, 1, g, w);
+    k_rns_balance<<<dim3((max_k + 31) / 32, ndesc), 256, 0, s>>>(d_desc, mode, g, w);
+    launches += 2;
+  }
   if (!a_presplit) {
     if (mode == kTN)
-      k_rns_scale_cols<<<dim3(max_m, ndesc), 256, 0, s>>>(d_desc, mode, 0, g, w);
+      k_rns_scale_cols<false><<<dim3(max_m, ndesc), 256, 0, s>>>(d_desc, mode, 0, g, w);
     else
       k_rns_scale_rows<<<dim3((max_m + 63) / 64, ndesc), 256, 0, s>>>(d_desc, mode, g, w);
     const unsigned gx = std::max(1u, std::min(chunks, 148u * 16 / (unsigned)std::max(1, g.a_mt * ndesc) + 1));
-    k_rns_split<<<dim3(gx, g.a_mt, ndesc), 2 * kTileM, 0, s>>>(d_desc, mode, 0, g, w);
+    split(gx, g.a_mt, 2 * kTileM, 0);
     launches += 2;
   }
-  k_rns_scale_cols<<<dim3(max_n, ndesc), 256, 0, s>>>(d_desc, mode, 1, g, w);
+  if (g.bal_off)
+    k_rns_scale_cols<true><<<dim3(max_n, ndesc), 256, 0, s>>>(d_desc, mode, 1, g, w);
+  else
+    k_rns_scale_cols<false><<<dim3(max_n, ndesc), 256, 0, s>>>(d_desc, mode, 1, g, w);
   {
     const unsigned gx = std::max(1u, std::min(chunks, 148u * 8 / (unsigned)std::max(1, g.nt * ndesc) + 1));
-    k_rns_split<<<dim3(gx, g.nt, ndesc), 2 * g.trb, 0, s>>>(d_desc, mode, 1, g, w);
+    split(gx, g.nt, 2 * g.trb, 1);
   }
   const int kper = (int)std::min<int64_t>(max_k, (int64_t)kTileK * ((g.ktc + g.ksplit - 1) / g.ksplit));
   if ((int64_t)kper * 121 * 121 < (1 << 24))

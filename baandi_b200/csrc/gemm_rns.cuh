@@ -19,12 +19,26 @@
 //   4. the Chinese remainder theorem returns the integer of each output from its residues as
 //      a fraction of the moduli's product (to 2^-74), which is scaled back to FP64.
 // Cauchy-Schwarz bounds every output by the product of the two norms, 2^(2 kNormBits), below
-// half the moduli's product, so no output can wrap.  The only rounding is that of step 1 and
-// of the final FP64 value: an output's error is about 2^-59 of the two norms' product, below
-// the FP64 summation's own.  Measured against 80-bit sums (2-norm, random operands), here and
-// for an FP64 GEMM: 864 x 480 x 80,725 A^H B 5.2e-16 and 7.7e-15 (2.0e-16 and 1.0e-14 with rows
-// falling by e^12), 80,725 x 480 x 864 A B 1.0e-16 and 1.4e-15, 129 x 16 x 1,000 1.0e-16 and
-// 3.7e-16.  Results do not depend on the K split or the launch shape: sums are exact.
+// half the moduli's product, so no output can wrap.  The only rounding is that of step 1, of the
+// fraction and of the final FP64 value.  Sums over K are exact; a different K split (it follows
+// from the launch's products and workspace) gives other representatives of the same residues and
+// with them other last bits of the fraction.
+//
+// The error is norm-wise: an output is off by about 2^-58 of its row's norm times its column's,
+// where an FP64 GEMM is off by a few 2^-53 of sum |a_k| |b_k|.  Taken over a result this is the
+// smaller one.  Against 80-bit sums (2-norm, random operands), here and for an FP64 GEMM: 864 x
+// 480 x 80,725 A^H B 5.2e-16 and 7.7e-15 (2.0e-16 and 1.0e-14 with rows falling by e^12), 80,725 x
+// 480 x 864 A B 1.0e-16 and 1.4e-15, 129 x 16 x 1,000 1.0e-16 and 3.7e-16.  An operand's entries
+// below 2^-5 of their row's norm keep fewer than 53 bits, so an output far below the product of
+// the norms can be less exact than an FP64 GEMM's: where a row and a column are graded against
+// each other.  Rotations have such rows (steep tails of Ritz vectors beside slow tails of
+// corrections, joined by small coefficients), so where A is split in the launch of an A B
+// product, K is balanced first (k_rns_balance).  Steep and slow tails (e^-q2 and (1 + q2)^-2, q2 to
+// 30), coefficients of 1e-8, largest error over sum |a_k| |b_k|: 7e-11 unbalanced, 2e-17 balanced,
+// 3e-16 in an FP64 GEMM; with coefficients from 1e-9 to 0.1, column by column, the median relative
+// error is 7e-15, 6e-16 and 3e-16, and entries 1e-12 below their row's largest stay less exact here
+// (relative 2e-8 against 1e-13).  The balance costs 0.3 % of the Si216 eigenproblem (143.4 -> 143.8
+// ms).  One more modulus (three more bits) made it 5 % slower and was not kept.
 //
 // Si216's projection (864 x 480 x 80,725, P split at build) takes 1.52 ms against the FP64 tiles'
 // 9.62 ms: 0.12 ms scales and 0.49 ms residues of x (3.8 TB/s), 0.87 ms products (56 % of the

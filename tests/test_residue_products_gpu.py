@@ -1,11 +1,14 @@
 """FP64 products on the int8 tensor cores (csrc/gemm_rns.cu) against extended-precision sums:
-tile edges, K remainders, every op, split and unsplit A, badly scaled and non-finite input.
+tile edges, K remainders, every op, split and unsplit A, several products in one launch, badly
+scaled, graded and non-finite input.
 
 Bound of an entry: a row is scaled by a power of two to a 2-norm of 2^57.3 .. 2^58.3 and
 every real part rounded to an integer, so each of its K complex values is off by at most
 2^-1/2 and, by Cauchy-Schwarz, the sum of K products by sqrt(K / 2) (1 / |a| + 1 / |b|) of the
 norms' product in scaled units: sqrt(2 K) 2^-57.3 |a| |b|.  The result is rounded to FP64
-twice more (2^-51 |c| covers that and the final addition).
+twice more (2^-51 |c| covers that and the final addition).  A B with A split in the launch
+takes the norms of A D and D^-1 B, D_k the power of two below max_j |B_kj| / |b_j| (real and
+imaginary parts apart, norms up to a factor of two): 4 |a D'| |b / D'| with D' that ratio itself.
 """
 from __future__ import annotations
 
@@ -42,10 +45,18 @@ def matrices(mode, m, n, k, seed):
     return a, z(n, k), z(n, m)
 
 
-def exact(mode, a, b):
-    """(n, m) product in 80-bit arithmetic and the bound's norm products."""
+def exact(mode, a, b, balanced=False, skip=()):
+    """(n, m) product in 80-bit arithmetic and the bound's norm products.  skip: columns of B that
+    the balance does not see (non-finite ones)."""
     left = (a.conj() if mode == 0 else a.T).astype(np.clongdouble)
-    norms = np.linalg.norm(b, axis=1)[:, None] * np.linalg.norm(np.abs(left).astype(np.float64), axis=1)[None, :]
+    la, lb = np.abs(left).astype(np.float64), np.abs(b)
+    factor = 1.0
+    if balanced and mode == 1:
+        parts, size = np.maximum(np.abs(b.real), np.abs(b.imag)), np.linalg.norm(b, axis=1)
+        rel = parts / np.where(size > 0.0, size, 1.0)[:, None]
+        d = np.maximum(np.max(np.delete(rel, list(skip), axis=0), axis=0), 2.0 ** -58)
+        la, lb, factor = la * d, lb / d, 4.0
+    norms = factor * np.linalg.norm(lb, axis=1)[:, None] * np.linalg.norm(la, axis=1)[None, :]
     return b.astype(np.clongdouble) @ left.T, norms
 
 
@@ -58,7 +69,7 @@ def test_tile_edges(mode, m, n, k):
     a[..., 0] *= 1e-3  # a graded row or column
     c = torch.from_numpy(c0.copy()).cuda()
     product(mode, torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), c, op, presplit)
-    want, norms = exact(mode, a, b)
+    want, norms = exact(mode, a, b, not presplit)
     if op == 1:
         want = c0 + want
     if op == 2:
@@ -77,7 +88,7 @@ def test_scales_and_nonfinite(mode, power):
     rows = a if mode == 0 else a.T          # row i of the left factor
     rows[2] = 0.0
     b[1] = 0.0
-    want, norms = exact(mode, a, b)
+    want, norms = exact(mode, a, b, True, skip=[3])
     ea, eb = np.zeros(m, np.int64), np.zeros(n, np.int64)
     ea[0], ea[1], eb[0] = power, -power, -power   # squares overflow and underflow; one product vanishes
     rows *= np.ldexp(1.0, ea)[:, None]
@@ -94,3 +105,23 @@ def test_scales_and_nonfinite(mode, power):
     w = np.ldexp(w.real, e) + 1j * np.ldexp(w.imag, e)
     bound = np.ldexp(np.sqrt(2 * k) * 2.0 ** -57.3 * norms[fine], e) + 2.0 ** -51 * np.abs(w) + 4 * np.finfo(np.float64).smallest_subnormal
     assert np.all(np.abs(got[fine] - w) <= bound)
+
+
+@pytest.mark.parametrize("steep", [0.35, 1.0])
+def test_graded_rotation(steep):
+    """Ritz vectors with steep tails and corrections with slow ones, rotated with coefficients of
+    order one and 1e-8: every entry within the FP64 sum's own bound, K 2^-53 (|A| |B|)."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(0)
+    m, n = 1500, 100
+    z = lambda *s: rng.standard_normal(s) + 1j * rng.standard_normal(s)
+    q2 = np.linspace(0.01, 30.0, m)
+    a = np.concatenate([z(n, m) * np.exp(-steep * q2), z(n, m) / (1.0 + q2) ** 2])
+    a /= np.linalg.norm(a, axis=1)[:, None]
+    b = np.concatenate([np.linalg.qr(z(n, n))[0], 1e-8 * z(n, n)], axis=1)
+    c = torch.zeros((n, m), dtype=torch.complex128, device="cuda")
+    product(1, torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), c, 0, 0)
+    want, _ = exact(1, a, b)
+    bound = 2 * n * 2.0 ** -53 * (np.abs(b) @ np.abs(a))
+    diff = np.abs((c.cpu().numpy() - want).astype(np.complex128))
+    assert np.all(diff <= bound), float(np.max(diff / bound))
