@@ -125,3 +125,41 @@ def test_graded_rotation(steep):
     bound = 2 * n * 2.0 ** -53 * (np.abs(b) @ np.abs(a))
     diff = np.abs((c.cpu().numpy() - want).astype(np.complex128))
     assert np.all(diff <= bound), float(np.max(diff / bound))
+
+
+@pytest.mark.parametrize("presplit", [0, 1])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_several_products(mode, presplit):
+    """Ragged products of one launch, empty slots among them, in a workspace made for larger ones
+    (fewer K splits than the products alone would take), as the Davidson's slots and k points."""
+    import torch
+    lib = L.load()
+    shapes = [(300, 96, 2100), (0, 0, 0), (129, 17, 4099), (513, 257, 70), (40, 1, 1300), (0, 5, 9), (256, 128, 64)]
+    rng = np.random.default_rng(11)
+    hosts, devs = [], []
+    for i, (m, n, k) in enumerate(shapes):
+        a, b, c = matrices(mode, max(m, 1), max(n, 1), max(k, 1), 40 + i)
+        a = a * np.exp(rng.uniform(-8, 8, a.shape[1]))[None, :] if i % 2 else a
+        hosts.append((a, b, c))
+        devs.append([torch.from_numpy(np.ascontiguousarray(t)).cuda() for t in (a, b, c)])
+    count = len(shapes)
+    ptrs = lambda j: (ctypes.c_void_p * count)(*[d[j].data_ptr() for d in devs])
+    lds = lambda j: (ctypes.c_int64 * count)(*[d[j].shape[1] for d in devs])
+    flat = (ctypes.c_int64 * (3 * count))(*[v for s in shapes for v in s])
+    for bounds in (None, (600, 300, 5000), (513, 257, 4100)):
+        bp = (ctypes.c_int64 * 3)(*bounds) if bounds else None
+        for d, h in zip(devs, hosts):
+            d[2].copy_(torch.from_numpy(h[2]))
+        rc = lib.bg_test_residue_products(mode, count, flat, ptrs(0), lds(0), ptrs(1), lds(1), ptrs(2), lds(2), 1,
+                                          presplit, bp, -1)
+        assert rc == 0
+        for (m, n, k), h, d in zip(shapes, hosts, devs):
+            got = d[2].cpu().numpy()
+            if m == 0 or n == 0 or k == 0:
+                assert np.array_equal(got, h[2])   # an empty slot's output is not touched
+                continue
+            want, norms = exact(mode, h[0], h[1], not presplit)
+            want = h[2] + want
+            diff = np.abs((got - want).astype(np.complex128))
+            bound = np.sqrt(2 * k) * 2.0 ** -57.3 * norms + 2.0 ** -51 * (np.abs(want).astype(np.float64) + np.abs(h[2]))
+            assert np.all(diff <= bound), ((m, n, k), float(np.max(diff / bound)))
