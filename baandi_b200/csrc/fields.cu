@@ -433,15 +433,18 @@ int bg_fields_lda_hartree(bg_fields* f, const double* density, double* v_hxc, do
   launch_chained(k_f_xc, kFieldBlocks, kFieldThreads, 0, f->stream, rho, total, f->vxc, f->work, f->part, f->err);
   for (int a = 2; a >= 0; --a) {
     const int blocks = (int)((total / b.n[a] + kLines - 1) / kLines);
-    launch_chained(k_f_lines<-1>, blocks, kFieldThreads, lines_smem(b.n[a]), f->stream, f->work, b, a, f->plan[a], f->tw[a]);
+    launch_chained(k_f_lines<-1>, blocks, kFieldThreads, lines_smem(b.n[a]), f->stream, f->work, b, a, f->plan[a],
+                   f->tw[a]);
   }
   launch_chained(k_f_poisson, kFieldBlocks, kFieldThreads, 0, f->stream, f->work, b, f->rc, 1.0 / (double)total);
   for (int a = 0; a < 3; ++a) {
     const int blocks = (int)((total / b.n[a] + kLines - 1) / kLines);
-    launch_chained(k_f_lines<1>, blocks, kFieldThreads, lines_smem(b.n[a]), f->stream, f->work, b, a, f->plan[a], f->tw[a]);
+    launch_chained(k_f_lines<1>, blocks, kFieldThreads, lines_smem(b.n[a]), f->stream, f->work, b, a, f->plan[a],
+                   f->tw[a]);
   }
   launch_chained(k_f_collect, kFieldBlocks, kFieldThreads, 0, f->stream, f->work, rho, f->vxc, total, vh, out, f->part);
-  launch_chained(k_f_energies, 1, kFieldThreads, 0, f->stream, f->part, kFieldBlocks, f->volume / (double)total, f->energies);
+  launch_chained(k_f_energies, 1, kFieldThreads, 0, f->stream, f->part, kFieldBlocks, f->volume / (double)total,
+                 f->energies);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
   if ((e = cudaMemcpyAsync(f->energies_host, f->energies, sizeof(double) * 3, cudaMemcpyDeviceToHost, f->stream)) !=
           cudaSuccess ||
@@ -495,9 +498,11 @@ static void f_transform(bg_fields* f, int sign) {
     const int a = sign < 0 ? 2 - i : i;
     const int blocks = (int)((b.total / b.n[a] + kLines - 1) / kLines);
     if (sign < 0)
-      launch_chained(k_f_lines<-1>, blocks, kFieldThreads, lines_smem(b.n[a]), f->stream, f->work, b, a, f->plan[a], f->tw[a]);
+      launch_chained(k_f_lines<-1>, blocks, kFieldThreads, lines_smem(b.n[a]), f->stream, f->work, b, a, f->plan[a],
+                     f->tw[a]);
     else
-      launch_chained(k_f_lines<1>, blocks, kFieldThreads, lines_smem(b.n[a]), f->stream, f->work, b, a, f->plan[a], f->tw[a]);
+      launch_chained(k_f_lines<1>, blocks, kFieldThreads, lines_smem(b.n[a]), f->stream, f->work, b, a, f->plan[a],
+                     f->tw[a]);
   }
 }
 

@@ -343,7 +343,8 @@ __device__ __forceinline__ void split_rows(const Operand& o, bool conj, int R, i
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       x[u] = make_double2(0.0, 0.0);
-      if (j < o.rows && k0 + u < o.K) x[u] = o.template balanced<BAL>(__ldg(o.X + (int64_t)(k0 + u) * o.sk + (int64_t)j * o.sj), k0 + u);
+      if (j < o.rows && k0 + u < o.K)
+        x[u] = o.template balanced<BAL>(__ldg(o.X + (int64_t)(k0 + u) * o.sk + (int64_t)j * o.sj), k0 + u);
     }
     unsigned al[8], ah[8], bl[8], bh[8];
 #pragma unroll
@@ -716,7 +717,8 @@ __global__ void __launch_bounds__(kMmaThreads, 1)
     __shared__ int s_none;
     if (tid == 0) {
       s_none = 0;
-      for (int t = s_consumed; t < s_issued; ++t) mbar_wait(smem_addr(&full[t % kStages]), (uint32_t)((t / kStages) & 1), &s_none, kWaitLimit);
+      for (int t = s_consumed; t < s_issued; ++t)
+        mbar_wait(smem_addr(&full[t % kStages]), (uint32_t)((t / kStages) & 1), &s_none, kWaitLimit);
       if (s_consumed > 0) {
         const int t = s_consumed - 1;
         mbar_wait(smem_addr(&empty[t % kStages]), (uint32_t)((t / kStages) & 1), &s_none, kWaitLimit);

@@ -856,8 +856,8 @@ static void density_planes(const OpTables* tabs, int gamma, const BoxGeo& g, con
   const size_t ds = density_smem_bytes(g);
   if constexpr (N != 0) {
     if (g.n0 == N && g.n1 == N) {
-      launch_chained(k_density_planes_fast<N>, dgrid, planes_threads<N, double2>(), ds, s, tabs, g, b, gamma, w, wstride, unit0,
-                                                                               part);
+      launch_chained(k_density_planes_fast<N>, dgrid, planes_threads<N, double2>(), ds, s, tabs, g, b, gamma, w,
+                     wstride, unit0, part);
       return;
     }
   }
@@ -896,7 +896,8 @@ int launch_density(const OpTables* tabs, int gamma, int max_groups, const BoxGeo
 #define BG_PLANES(NN) density_planes<NN>(tabs, gamma, g, b, weights, wstride, u0, part, dgrid, s)
     BG_DENS(BG_PLANES)
 #undef BG_PLANES
-    launch_chained(k_density_sum_chunks, dim3(bx, b.nk), 256, 0, s, part, n, total, volume, u0 == 0, u0 + n >= max_units, ksum);
+    launch_chained(k_density_sum_chunks, dim3(bx, b.nk), 256, 0, s, part, n, total, volume, u0 == 0,
+                   u0 + n >= max_units, ksum);
     launches += 2;
   }
 #undef BG_DENS
@@ -947,14 +948,19 @@ int launch_nonlocal(const NlDev* nl, int gamma, const NlShape& sh, int max_rows,
   if (gamma) {
     {
       StageScope sc(ev, 3, s);
-      launch_chained(k_project<double>, pg, 256, tiles::tn48m_smem_bytes<double>(), s, nl, sh.nproj, sh.ksplit, sh.kchunk, b);
+      launch_chained(k_project<double>, pg, 256, tiles::tn48m_smem_bytes<double>(), s, nl, sh.nproj, sh.ksplit,
+                     sh.kchunk, b);
     }
     { StageScope sc(ev, 4, s); launch_chained(k_couple<double>, cg, cth, 0, s, nl, sh.nproj, sh.ksplit, b); }
-    { StageScope sc(ev, 5, s); launch_chained(k_back<double>, bg_, 256, tiles::nn64m_smem_bytes<double>(), s, nl, sh.nproj, b); }
+    {
+      StageScope sc(ev, 5, s);
+      launch_chained(k_back<double>, bg_, 256, tiles::nn64m_smem_bytes<double>(), s, nl, sh.nproj, b);
+    }
   } else {
     {
       StageScope sc(ev, 3, s);
-      launch_chained(k_project<double2>, pg, 256, tiles::tn48m_smem_bytes<double2>(), s, nl, sh.nproj, sh.ksplit, sh.kchunk, b);
+      launch_chained(k_project<double2>, pg, 256, tiles::tn48m_smem_bytes<double2>(), s, nl, sh.nproj, sh.ksplit,
+                     sh.kchunk, b);
     }
     { StageScope sc(ev, 4, s); launch_chained(k_couple<double2>, cg, cth, 0, s, nl, sh.nproj, sh.ksplit, b); }
     {

@@ -1538,8 +1538,8 @@ class KsetSolver {
   static bool small(int cap) { return vec_smem(cap) + mat_smem(cap) <= 200 * 1024; }
   size_t ctl_smem() const { return vec_smem(o_.cap) + (o_.smem_matrices ? mat_smem(o_.cap) : 0); }
   int64_t ctl(int phase) {
-    launch_chained(k_dv_ctl<D>, nk_, kCtlThreads, ctl_smem(), s_, phase, d_bufs_, d_ctl_, d_nn_, d_tn_, d_cp_, d_dyn_, d_opts_,
-                                                     nk_, ks_->gamma);
+    launch_chained(k_dv_ctl<D>, nk_, kCtlThreads, ctl_smem(), s_, phase, d_bufs_, d_ctl_, d_nn_, d_tn_, d_cp_, d_dyn_,
+                   d_opts_, nk_, ks_->gamma);
     return 1;
   }
   // residues: large products go through the residue products (not in the repair, whose
@@ -1563,11 +1563,11 @@ class KsetSolver {
   int64_t tn(int nslots, bool residues = true) {
     const unsigned t = (unsigned)((o_.cap + 47) / 48);
     residues = residues && rns_work_;
-    launch_chained(k_dv_tn<D>, dim3(t, t, (unsigned)(nslots * nk_ * ksplit_)), 256, tiles::tn48m_smem_bytes<D>(), s_, 
-        d_bufs_, d_tn_, nk_, ksplit_, slot_elems_, residues ? 1 : 0);
+    launch_chained(k_dv_tn<D>, dim3(t, t, (unsigned)(nslots * nk_ * ksplit_)), 256, tiles::tn48m_smem_bytes<D>(), s_,
+                   d_bufs_, d_tn_, nk_, ksplit_, slot_elems_, residues ? 1 : 0);
     const unsigned blocks = (unsigned)std::min<int64_t>(((int64_t)o_.cap * o_.cap + 255) / 256, 64);
     launch_chained(k_dv_tn_sum<D>, dim3(blocks, 1, (unsigned)(nslots * nk_)), 256, 0, s_, d_bufs_, d_tn_, nk_, ksplit_,
-                                                                              slot_elems_, residues ? 1 : 0);
+                   slot_elems_, residues ? 1 : 0);
     int64_t l = 2;
     if (residues) {
       launch_chained(k_dv_rns_descs<D>, 1, 128, 0, s_, d_bufs_, d_nn_, 0, d_tn_, nslots, nk_, d_rns_);
@@ -1664,8 +1664,8 @@ class KsetSolver {
     return 1;
   }
   int64_t corr() {
-    launch_chained(k_dv_corrections<D>, dim3((unsigned)o_.n, (unsigned)nk_), 256, 0, s_, 
-        d_bufs_, d_ctl_, d_opts_, static_cast<const __nv_bfloat16*>(ks_->ctx->learned));
+    launch_chained(k_dv_corrections<D>, dim3((unsigned)o_.n, (unsigned)nk_), 256, 0, s_, d_bufs_, d_ctl_, d_opts_,
+                   static_cast<const __nv_bfloat16*>(ks_->ctx->learned));
     return 1;
   }
   // Many-block reduced problem (wide_rr.cuh): extension of the factor, then the

@@ -359,8 +359,9 @@ int bg_mixer_update(bg_mixer* m, const double* x, const double* f, double* next,
   const int slot = it > 1 ? (it - 2) % m->history : -1;
   const int p = std::min(std::max(it - 1, 0), m->history);
   const unsigned gb = grid_for(n);
-  launch_chained(k_mix_diff, gb, 256, 0, m->stream, dxp, dfp, m->prev_x, m->prev_f, m->dx + (slot < 0 ? 0 : (int64_t)slot * n),
-                                        m->df + (slot < 0 ? 0 : (int64_t)slot * n), n, slot >= 0 ? 1 : 0);
+  launch_chained(k_mix_diff, gb, 256, 0, m->stream, dxp, dfp, m->prev_x, m->prev_f,
+                 m->dx + (slot < 0 ? 0 : (int64_t)slot * n), m->df + (slot < 0 ? 0 : (int64_t)slot * n), n,
+                 slot >= 0 ? 1 : 0);
   if (p > 0) {
     launch_chained(k_mix_forms, p * (p + 1) / 2 + p, kMixThreads, 0, m->stream, m->df, n, p, dfp, m->w, m->forms);
     launch_chained(k_mix_solve, 1, 32, 0, m->stream, m->forms, p, m->gamma, m->out);
@@ -383,8 +384,8 @@ int bg_mixer_update(bg_mixer* m, const double* x, const double* f, double* next,
       return fail(ctx, BG_EINVAL, msg);
     }
   }
-  launch_chained(k_mix_apply, gb, 256, 0, m->stream, dxp, dfp, m->dx, m->df, n, p, m->gamma, m->smooth, m->screening, m->beta,
-                                         dnext, m->reduced, m->err);
+  launch_chained(k_mix_apply, gb, 256, 0, m->stream, dxp, dfp, m->dx, m->df, n, p, m->gamma, m->smooth, m->screening,
+                 m->beta, dnext, m->reduced, m->err);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(ctx, e, "kernel launch");
   if (ptr_kind == BG_PTR_HOST && (e = cudaMemcpyAsync(next, dnext, bytes, cudaMemcpyDeviceToHost, m->stream)) != cudaSuccess)
     return cuda_fail(ctx, e, "copy out");

@@ -152,9 +152,11 @@ void launch_planes_any(const OpTables* tabs, const BoxGeo& g, const Batch& b, di
 void launch_density_any(const OpTables* tabs, const BoxGeo& g, const Batch& b, int gamma, const double* w, int wstride,
                         int unit0, double* part, dim3 grid, cudaStream_t s) {
   if (any_warps(g) == 8)
-    launch_chained(k_density_planes_any<8>, grid, 256, any_smem(g, false), s, tabs, g, b, gamma, w, wstride, unit0, part);
+    launch_chained(k_density_planes_any<8>, grid, 256, any_smem(g, false), s, tabs, g, b, gamma, w, wstride, unit0,
+                   part);
   else
-    launch_chained(k_density_planes_any<16>, grid, 512, any_smem(g, false), s, tabs, g, b, gamma, w, wstride, unit0, part);
+    launch_chained(k_density_planes_any<16>, grid, 512, any_smem(g, false), s, tabs, g, b, gamma, w, wstride, unit0,
+                   part);
 }
 
 int configure_planes_any() {

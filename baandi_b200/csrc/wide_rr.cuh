@@ -817,8 +817,9 @@ __global__ void __launch_bounds__(kT) k_w_tri_gs(const Bufs<D>* __restrict__ buf
   }
 }
 
-// Y[:, c] = H_0 H_1 ... H_{m-3} (s . Z[:, order[c]]) for c < m: `cols` columns per block, one warp per column; each reflector is staged once per block in shared memory
-// (double-buffered, one barrier per reflector) and applied by every warp to its column.
+// Y[:, c] = H_0 H_1 ... H_{m-3} (s . Z[:, order[c]]) for c < m: `cols` columns per block, one warp
+// per column; each reflector is staged once per block in shared memory (double-buffered, one
+// barrier per reflector) and applied by every warp to its column.
 template <class D>
 __global__ void __launch_bounds__(kT) k_w_back(const Bufs<D>* __restrict__ bufs, const Ctl* __restrict__ ctl, int cap,
                                                int cols) {
