@@ -40,10 +40,10 @@
 // (relative 2e-8 against 1e-13).  The balance costs 0.3 % of the Si216 eigenproblem (143.4 -> 143.8
 // ms).  One more modulus (three more bits) made it 5 % slower and was not kept.
 //
-// Si216's projection (864 x 480 x 80,725, P split at build) takes 1.52 ms against the FP64 tiles'
-// 9.62 ms: 0.12 ms scales and 0.49 ms residues of x (3.8 TB/s), 0.87 ms products (56 % of the
-// int8 peak, bound by the tiles' L2 traffic, 40 bytes per SM and cycle), 0.04 ms
-// reconstruction.  Its back-projection takes 1.96 against 8.69 ms: 1.07 ms products, 0.86 ms
+// Si216's projection (864 x 480 x 80,725, P split at build) takes 1.57 ms against the FP64 tiles'
+// 9.62 ms: 0.11 ms scales and 0.49 ms residues of x (3.8 TB/s), 0.93 ms products (52 % of the
+// int8 peak, bound by the tiles' L2 traffic, 40 bytes per SM and cycle), 0.03 ms
+// reconstruction.  Its back-projection takes 1.79 against 8.69 ms: 1.12 ms products, 0.65 ms
 // reconstruction (1.2 GB of residues read, y read and written).
 #pragma once
 
